@@ -97,6 +97,27 @@ struct SweepPlan {
    // strand's warp never overwrites a ring slot still to be read
    DBuf<int32_t> seg_keep;
 };
+
+// Wavefront plan of one sweep direction (see wave.cu): lines in groups of up
+// to 32, the coefficients in the order the steps read them.
+constexpr int kWaveExt = 4;        // entries a row may have in earlier groups
+// The wavefront is taken when a line has at least kWaveMinLine rows on
+// average and a step at least kWaveMinLanes active lanes.
+constexpr int64_t kWaveMinLine = 8;
+constexpr int64_t kWaveMinLanes = 4;
+struct WavePlan {
+   bool on = false, fwd = true;
+   bool ext = false;          // some row has entries in earlier groups
+   bool clean = false;        // equal lines, one step apart
+   int ngroups = 0;
+   int64_t tiles = 0;         // 32-step layout tiles
+   DBuf<int32_t> line, shift, dshift, eoff;
+   DBuf<int32_t> g_line, g_tile, g_nch, g_edge, g_sm1, tile_g;
+   DBuf<double> coef, ecoef;  // step order; ecoef: natural order
+   DBuf<double> edge;         // last lines of the groups on their way to the next group
+   DBuf<double> gdot;
+   DBuf<int> ticket;
+};
 }  // namespace ofg
 
 namespace ofg {
@@ -113,6 +134,7 @@ struct ofg_prec {
    ofg::DBuf<double> t;
    ofg::DBuf<int> status;    // bounded-wait failures (bit 0: timeout, bit 1: wave)
    ofg::SweepPlan fwd, bwd;
+   ofg::WavePlan wfwd, wbwd;  // both on, or both off
    ofg::DBuf<int32_t> tpos;  // D-ILU: transposed position of each lower entry
    ofg::DBuf<double> dot;    // (r, z) of the last backward sweep that was asked for it
    int grid = 0;             // blocks of the persistent factorisation sweep launch
@@ -173,6 +195,16 @@ void check_status(ofg_prec* P);
 // that IEEE arithmetic never produces (results are the canonical NaN).
 constexpr unsigned long long kSentinelBits = 0x7FF4DEADBEEF0001ULL;
 void fill_sentinel(double* p, int64_t n);
+
+// wave.cu: the wavefront plan of a direction (chain: row rho depends on
+// row rho - 1, logical order; tpos: transposed positions when a
+// factorisation is wanted); false when the matrix has no such lines
+bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpos, WavePlan& p);
+void wave_factor(ofg_prec* P);                // D-ILU pivots of the current values
+void wave_values(ofg_prec* P, WavePlan& p);   // the plan's copy of values and pivots
+void wave_solve(ofg_prec* P, bool fwd, const double* in, double* out, double* reset,
+                const double* dot_with, double* dot_out, const int* skip);
+void wave_repair(WavePlan& p);                // after a wait ran out
 
 // learned.cu: run the network on the matrix's current values and rebuild
 // G / G^T; z = G^T G r in FP64 (r and z may alias; rz as above when they

@@ -933,9 +933,8 @@ void fill_sentinel(double* p, int64_t n)
 
 namespace {
 
-// Strands start where a row does not depend on its predecessor; runs shorter
-// than kMinStrand are merged forward, runs longer than kMaxStrand are split.
-void build_plan(ofg_matrix* A, bool fwd, SweepPlan& plan)
+// chain[rho]: logical row rho depends on the row before it
+std::vector<int8_t> host_chain(ofg_matrix* A, bool fwd)
 {
    const int64_t n = A->n;
    DBuf<int8_t> chain(n > 0 ? n : 1);
@@ -945,7 +944,14 @@ void build_plan(ofg_matrix* A, bool fwd, SweepPlan& plan)
       count_launch();
       OFG_LAUNCH_CHECK();
    }
-   std::vector<int8_t> c = chain.to_host(n);
+   return chain.to_host(n);
+}
+
+// Strands start where a row does not depend on its predecessor; runs shorter
+// than kMinStrand are merged forward, runs longer than kMaxStrand are split.
+void build_plan(ofg_matrix* A, bool fwd, const std::vector<int8_t>& c, SweepPlan& plan)
+{
+   const int64_t n = A->n;
    std::vector<int32_t> starts;
    int64_t cur = 0;
    for (int64_t r = 1; r <= n; ++r) {
@@ -1144,6 +1150,8 @@ void check_status(ofg_prec* P)
    P->status.download(&h, 1);
    if (h) {
       P->status.zero();
+      wave_repair(P->wfwd);
+      wave_repair(P->wbwd);
       throw Error(OFG_ERR_TIMEOUT, "triangular sweep wait ran out (status " + std::to_string(h) + ")");
    }
 }
@@ -1178,34 +1186,51 @@ void prec_setup(ofg_prec* P)
       throw Error(OFG_ERR_PIVOT, "zero pivot detected in row " + std::to_string(h + 1));
    if (P->type == OFG_DIAG) return;
 
-   if (!P->fwd.start.p) {
-      int per_sm = 0;
-      OFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<FWD_DILU>,
-                                                             kWarpsPerBlock * 32, 0));
-      P->grid = std::max(1, per_sm) * num_sms();
-      OFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_sweep<FWD_DILU, 8>,
-                                                             kBandWarps * 32, 0));
-      P->solve_grid = std::max(1, per_sm) * num_sms();
-      build_plan(A, true, P->fwd);
-      build_plan(A, false, P->bwd);
+   const bool ilu = P->type == OFG_DILU || P->type == OFG_ILU;
+   if (ilu && !P->tpos.p) {
+      P->tpos.alloc(A->nnz > 0 ? A->nnz : 1);
+      if (n) {
+         transpose_positions<<<grid_for(n, 256), 256, 0, stream()>>>(n, A->row_ptr.p, A->col.p,
+                                                                     A->dpos.p, P->tpos.p);
+         count_launch();
+         OFG_LAUNCH_CHECK();
+      }
+   }
+   if (!P->status.p) {
       P->status.alloc(1);
       P->t.alloc(n > 0 ? n : 1);
       P->dot.alloc(1);
+      const std::vector<int8_t> cf = host_chain(A, true), cb = host_chain(A, false);
+      const bool wave = wave_build(A, true, cf.data(), ilu ? P->tpos.p : nullptr, P->wfwd) &&
+                        wave_build(A, false, cb.data(), nullptr, P->wbwd);
+      if (!wave) {
+         P->wfwd = WavePlan();
+         P->wbwd = WavePlan();
+         int per_sm = 0;
+         OFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<FACTOR>,
+                                                                kWarpsPerBlock * 32, 0));
+         P->grid = std::max(1, per_sm) * num_sms();
+         OFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_sweep<FWD_DILU, 8>,
+                                                                kBandWarps * 32, 0));
+         P->solve_grid = std::max(1, per_sm) * num_sms();
+         build_plan(A, true, cf, P->fwd);
+         build_plan(A, false, cb, P->bwd);
+      }
    }
    P->status.zero();
    fill_sentinel(P->t.p, n);
+   if (P->wfwd.on) {
+      if (ilu) {
+         wave_factor(P);
+         check_status(P);
+      }
+      wave_values(P, P->wfwd);
+      wave_values(P, P->wbwd);
+      return;
+   }
    fill_slot_values(A, P->fwd);
    fill_slot_values(A, P->bwd);
-   if (P->type == OFG_DILU || P->type == OFG_ILU) {
-      if (!P->tpos.p) {
-         P->tpos.alloc(A->nnz > 0 ? A->nnz : 1);
-         if (n) {
-            transpose_positions<<<grid_for(n, 256), 256, 0, stream()>>>(n, A->row_ptr.p, A->col.p,
-                                                                        A->dpos.p, P->tpos.p);
-            count_launch();
-            OFG_LAUNCH_CHECK();
-         }
-      }
+   if (ilu) {
       // pivots = 1/(a_ll - sum a_li pinv_i a_il), rows in natural order
       fill_sentinel(P->pivot.p, n);
       SweepArgs g = base_args(P, P->fwd);
@@ -1233,6 +1258,14 @@ void prec_apply_device(ofg_prec* P, const double* r, double* z, double* rz, cons
          return;
       case OFG_LEARNED: learned_apply(P, r, z, rz, skip); return;
       default: break;
+   }
+   if (P->wfwd.on) {
+      // (the results of a sweep are waited for in memory only with E slots:
+      // then each sweep clears the other's buffer)
+      wave_solve(P, true, r, P->t.p, P->wbwd.ext ? z : nullptr, nullptr, nullptr, skip);
+      const bool dot = rz && r != z;
+      wave_solve(P, false, P->t.p, z, P->wfwd.ext ? P->t.p : nullptr, dot ? r : nullptr, rz, skip);
+      return;
    }
    const bool dilu = (P->type != OFG_SSOR);
    // forward: t = L-solve(r); clears z for the backward sweep
