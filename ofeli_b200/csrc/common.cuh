@@ -193,12 +193,13 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 template <typename... KArgs, typename... Args>
-void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, Args... args)
+void launch_pdl_smem(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                     Args... args)
 {
    cudaLaunchConfig_t cfg = {};
    cfg.gridDim = dim3(grid);
    cfg.blockDim = dim3(block);
-   cfg.dynamicSmemBytes = 0;
+   cfg.dynamicSmemBytes = smem;
    cfg.stream = stream();
    cudaLaunchAttribute attr[1];
    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -207,6 +208,12 @@ void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, Args...
    cfg.numAttrs = 1;
    OFG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
    count_launch();
+}
+
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, Args... args)
+{
+   launch_pdl_smem(kernel, grid, block, 0, args...);
 }
 
 inline unsigned grid_for(int64_t work, int block, int max_blocks_per_sm = 8)

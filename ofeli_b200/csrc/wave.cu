@@ -481,8 +481,6 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
    using Sh = WaveShared<MODE>;
    extern __shared__ __align__(128) unsigned char wave_raw[];
    Sh& sh = *reinterpret_cast<Sh*>(wave_raw);
-   if (g.skip && *g.skip) return;
-   prof_mark(g.worked);
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    const int n = (int)g.n;
    if (threadIdx.x == 0) {
@@ -501,6 +499,13 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
       (&sh.z[0][0])[i] = wave_sentinel();
    for (int i = threadIdx.x; i < Sh::NT * kTileChunks * kWaveF / 2 * kWaveCPitch; i += blockDim.x)
       (&sh.c[0][0])[i] = wave_sentinel();
+   // the kernel before may still be running up to here (programmatic dependent
+   // launch); the next one may set itself up from here on, when every block
+   // of this grid has started
+   pdl_wait();
+   pdl_release();
+   if (g.skip && *g.skip) return;
+   prof_mark(g.worked);
    unsigned tiles = 0;  // of the groups before this one: place and phase of every role
    for (;;) {
       __syncthreads();
@@ -1059,9 +1064,7 @@ void launch_wave(const WaveArgs& g)
    OFG_CUDA(cudaFuncSetAttribute(wave_sweep<MODE, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
    const int blocks = std::min(g.ngroups, num_sms());
-   wave_sweep<MODE, EXT><<<blocks, wave_threads(EXT), smem, stream()>>>(g);
-   count_launch();
-   OFG_LAUNCH_CHECK();
+   launch_pdl_smem(wave_sweep<MODE, EXT>, (unsigned)blocks, (unsigned)wave_threads(EXT), smem, g);
 }
 
 template <int MODE>
