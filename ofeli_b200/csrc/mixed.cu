@@ -157,7 +157,7 @@ __device__ __forceinline__ bool decide_pause(MixState* S, double rr2, int it, co
 // q = A p over four rows per thread; (p, q) left as per-block partials for
 // mx_update.  UNI: slices with uniform offsets (suni[s] >= 0) read one
 // offset per position from stab and gather p with vector loads.
-template <class T, class I, bool UNI = false>
+template <class T, class I, bool UNI = false, bool VAL = false>
 __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) mx_spmv(int64_t nquads, const int32_t* __restrict__ sp,
                                                      const I* __restrict__ scol,
                                                      const T* __restrict__ sval,
@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) mx_spmv(int64_t nquads
                                                      float* __restrict__ q, const MixState* S,
                                                      double* pq, int* worked,
                                                      const int32_t* __restrict__ suni = nullptr,
-                                                     const int16_t* __restrict__ stab = nullptr)
+                                                     const int16_t* __restrict__ stab = nullptr,
+                                                     ValueTab vt = ValueTab())
 {
    pdl_wait();
    pdl_release();
@@ -177,8 +178,14 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) mx_spmv(int64_t nquads
       const int64_t r0 = t * 4;
       const int64_t s = r0 >> 5;
       const int lane0 = (int)(r0 & 31);
-      const int32_t beg = sp[s], w = (sp[s + 1] - beg) >> 5;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      int2 hd = make_int2(-1, 0);
+      if (VAL) hd = __ldg(vt.head + s);
+      if (VAL && hd.x >= 0) {
+         acc = value_quad(vt.tab + hd.x, hd.y, p, (int)r0);
+      }
+      else {
+      const int32_t beg = sp[s], w = (sp[s + 1] - beg) >> 5;
       const T* vp = sval + beg + lane0;
       const int32_t u = UNI ? suni[s] : -1;
       if (u >= 0) {
@@ -204,6 +211,7 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) mx_spmv(int64_t nquads
 #pragma unroll 8
             for (int32_t k = 0; k < w; ++k) step(k);
          }
+      }
       }
       *reinterpret_cast<float4*>(q + r0) = acc;
       const float4 pr = *reinterpret_cast<const float4*>(p + r0);
@@ -308,7 +316,7 @@ __global__ void __launch_bounds__(kRedBlock, 8) mx_direction(int64_t nquads,
 
 // After iteration `it` (decide): the stop decision from mx_update's
 // partials; then t = G r
-template <class V, class I, bool UNI = false>
+template <class V, class I, bool UNI = false, bool VAL = false>
 __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_lower(int64_t nquads, const int32_t* __restrict__ sp,
                                                       const I* __restrict__ scol,
                                                       const V* __restrict__ sval,
@@ -316,7 +324,8 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_lower(int64_t nquad
                                                       MixState* S, const double* __restrict__ rpart,
                                                       int it, int decide, StopRule st, int* worked,
                                                       const int32_t* __restrict__ suni = nullptr,
-                                                      const int16_t* __restrict__ stab = nullptr)
+                                                      const int16_t* __restrict__ stab = nullptr,
+                                                      ValueTab vt = ValueTab())
 {
    pdl_wait();
    pdl_release();
@@ -330,11 +339,11 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_lower(int64_t nquad
    int64_t stride = (int64_t)gridDim.x * blockDim.x;
    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nquads; i += stride)
       *reinterpret_cast<float4*>(t + i * 4) =
-         sell_quad<V, I, UNI>(sp, scol, sval, r, i * 4, suni, stab);
+         sell_quad<V, I, UNI, VAL>(sp, scol, sval, r, i * 4, suni, stab, vt);
 }
 
 // z = G^T t; (r, z) left as partials for lg_direction
-template <class V, class I, bool UNI = false>
+template <class V, class I, bool UNI = false, bool VAL = false>
 __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_upper(int64_t nquads, const int32_t* __restrict__ sp,
                                                       const I* __restrict__ scol,
                                                       const V* __restrict__ sval,
@@ -342,7 +351,8 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_upper(int64_t nquad
                                                       const float* __restrict__ r, const MixState* S,
                                                       double* cpart, int* worked,
                                                       const int32_t* __restrict__ suni = nullptr,
-                                                      const int16_t* __restrict__ stab = nullptr)
+                                                      const int16_t* __restrict__ stab = nullptr,
+                                                      ValueTab vt = ValueTab())
 {
    pdl_wait();
    pdl_release();
@@ -351,7 +361,7 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) lg_upper(int64_t nquad
    double v[1] = {0.0};
    int64_t stride = (int64_t)gridDim.x * blockDim.x;
    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nquads; i += stride) {
-      const float4 zi = sell_quad<V, I, UNI>(sp, scol, sval, t, i * 4, suni, stab);
+      const float4 zi = sell_quad<V, I, UNI, VAL>(sp, scol, sval, t, i * 4, suni, stab, vt);
       *reinterpret_cast<float4*>(z + i * 4) = zi;
       const float4 ri = *reinterpret_cast<const float4*>(r + i * 4);
       v[0] += (double)ri.x * zi.x + (double)ri.y * zi.y + (double)ri.z * zi.z + (double)ri.w * zi.w;
@@ -455,6 +465,28 @@ bool mostly_uniform(const ofg_matrix* M)
    return M->utab_len > 0 && M->uni_nnz >= 0.9 * (double)M->nnz;
 }
 
+// The value tables of one matrix for one solve (see ValueTab)
+struct SliceValues {
+   DBuf<int2> head, tab;
+   template <class V>
+   void scan(const ofg_matrix* M, const V* vals, unsigned long long* count)
+   {
+      head.alloc(M->nslices);
+      tab.alloc(M->utab_len);
+      scan_slice_values<<<(unsigned)((M->nslices * 32 + 255) / 256), 256, 0, stream()>>>(
+         M->nslices, M->sell_ptr.p, vals, M->sell_uni.p, M->sell_utab.p, head.p, tab.p, count);
+      count_launch();
+      OFG_LAUNCH_CHECK();
+   }
+   ValueTab get() const { return ValueTab{head.p, tab.p}; }
+};
+
+// Worth it from half of the entries on
+bool mostly_shared(const ofg_matrix* M, unsigned long long shared)
+{
+   return 2 * shared >= (unsigned long long)M->nnz;
+}
+
 }  // namespace
 
 void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const double* b, double* x,
@@ -537,8 +569,21 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
    inv_diag32<<<grid_for(nv, 256), 256, 0, stream()>>>(n, npad, A->dpos.p, A->val.p, dinv.p,
                                                         prec_type == OFG_IDENT ? 1 : 0, bad.p);
    count_launch();
+   // slices that share their values, in A (not in the lossy BF16 copy), G, G^T
+   SliceValues av, lv, uv;
+   DBuf<unsigned long long> shared(3);
+   shared.zero();
+   if (auni && inner_bits != 16) av.scan(A, A->sell_val.p, shared.p);
+   using bf16 = __nv_bfloat16;
+   if (luni) lv.scan(LP->gl, reinterpret_cast<const bf16*>(LP->gl->sell_valbf.p), shared.p + 1);
+   if (uuni) uv.scan(LP->gu, reinterpret_cast<const bf16*>(LP->gu->sell_valbf.p), shared.p + 2);
    int hb[2] = {0, 0};
+   unsigned long long hs[3] = {0, 0, 0};
+   OFG_CUDA(cudaMemcpyAsync(hs, shared.p, sizeof(hs), cudaMemcpyDeviceToHost, stream()));
    bad.download(hb, 2);
+   const bool aval = auni && inner_bits != 16 && mostly_shared(A, hs[0]);
+   const bool lval = luni && mostly_shared(LP->gl, hs[1]);
+   const bool uval = uuni && mostly_shared(LP->gu, hs[2]);
    OFG_REQUIRE(!hb[0], OFG_ERR_PIVOT, "zero diagonal entry");
    int bits = inner_bits;
    if (inner_bits == 0) {
@@ -576,32 +621,40 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
       const bf* vl = reinterpret_cast<const bf*>(learned ? LP->gl->sell_valbf.p : nullptr);
       const bf* vu = reinterpret_cast<const bf*>(learned ? LP->gu->sell_valbf.p : nullptr);
       int* worked = prof_begin();
-      if (luni)
+      if (lval)
+         launch_pdl(lg_lower<bf, int16_t, true, true>, gq, kRedBlock, nquads, LP->gl->sell_ptr.p,
+                    LP->gl->sell_d16.p, vl, rr.p, tz.p, S.p, rpart, it, decide, st, worked,
+                    LP->gl->sell_uni.p, LP->gl->sell_utab.p, lv.get());
+      else if (luni)
          launch_pdl(lg_lower<bf, int16_t, true>, gq, kRedBlock, nquads, LP->gl->sell_ptr.p,
                     LP->gl->sell_d16.p, vl, rr.p, tz.p, S.p, rpart, it, decide, st, worked,
-                    LP->gl->sell_uni.p, LP->gl->sell_utab.p);
+                    LP->gl->sell_uni.p, LP->gl->sell_utab.p, ValueTab());
       else if (g16)
          launch_pdl(lg_lower<bf, int16_t>, gq, kRedBlock, nquads, LP->gl->sell_ptr.p,
                     LP->gl->sell_d16.p, vl, rr.p, tz.p, S.p, rpart, it, decide, st, worked,
-                    nullptr, nullptr);
+                    nullptr, nullptr, ValueTab());
       else
          launch_pdl(lg_lower<bf, int32_t>, gq, kRedBlock, nquads, LP->gl->sell_ptr.p,
                     LP->gl->sell_col.p, vl, rr.p, tz.p, S.p, rpart, it, decide, st, worked,
-                    nullptr, nullptr);
+                    nullptr, nullptr, ValueTab());
       prof_end(PROF_LEARNED_APPLY, gl_bytes + 8.0 * n);
       worked = prof_begin();
-      if (uuni)
+      if (uval)
+         launch_pdl(lg_upper<bf, int16_t, true, true>, gq, kRedBlock, nquads, LP->gu->sell_ptr.p,
+                    LP->gu->sell_d16.p, vu, tz.p, zz.p, rr.p, S.p, cpart, worked,
+                    LP->gu->sell_uni.p, LP->gu->sell_utab.p, uv.get());
+      else if (uuni)
          launch_pdl(lg_upper<bf, int16_t, true>, gq, kRedBlock, nquads, LP->gu->sell_ptr.p,
                     LP->gu->sell_d16.p, vu, tz.p, zz.p, rr.p, S.p, cpart, worked,
-                    LP->gu->sell_uni.p, LP->gu->sell_utab.p);
+                    LP->gu->sell_uni.p, LP->gu->sell_utab.p, ValueTab());
       else if (g16)
          launch_pdl(lg_upper<bf, int16_t>, gq, kRedBlock, nquads, LP->gu->sell_ptr.p,
                     LP->gu->sell_d16.p, vu, tz.p, zz.p, rr.p, S.p, cpart, worked, nullptr,
-                    nullptr);
+                    nullptr, ValueTab());
       else
          launch_pdl(lg_upper<bf, int32_t>, gq, kRedBlock, nquads, LP->gu->sell_ptr.p,
                     LP->gu->sell_col.p, vu, tz.p, zz.p, rr.p, S.p, cpart, worked, nullptr,
-                    nullptr);
+                    nullptr, ValueTab());
       prof_end(PROF_LEARNED_APPLY, gu_bytes + 12.0 * n);
       launch_pdl(lg_direction, gq, kRedBlock, nquads, zz.p, p.p, d.p, upd_d, S.p, cpart, it, fresh);
    };
@@ -651,27 +704,38 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
             int* worked = prof_begin();
             const int32_t* su = A->sell_uni.p;
             const int16_t* st16 = A->sell_utab.p;
-            if (bits == 32 && auni)
+            if (aval && bits == 32)
+               launch_pdl(mx_spmv<float, int16_t, true, true>, gq, kRedBlock, nquads,
+                          A->sell_ptr.p, A->sell_d16.p, A->sell_val32.p, p.p, q.p, S.p, pq, worked,
+                          su, st16, av.get());
+            else if (aval)
+               launch_pdl(mx_spmv<__nv_bfloat16, int16_t, true, true>, gq, kRedBlock, nquads,
+                          A->sell_ptr.p, A->sell_d16.p, v16.p, p.p, q.p, S.p, pq, worked, su, st16,
+                          av.get());
+            else if (bits == 32 && auni)
                launch_pdl(mx_spmv<float, int16_t, true>, gq, kRedBlock, nquads, A->sell_ptr.p,
-                          A->sell_d16.p, A->sell_val32.p, p.p, q.p, S.p, pq, worked, su, st16);
+                          A->sell_d16.p, A->sell_val32.p, p.p, q.p, S.p, pq, worked, su, st16,
+                          ValueTab());
             else if (bits == 32 && a16)
                launch_pdl(mx_spmv<float, int16_t>, gq, kRedBlock, nquads, A->sell_ptr.p,
                           A->sell_d16.p, A->sell_val32.p, p.p, q.p, S.p, pq, worked, nullptr,
-                          nullptr);
+                          nullptr, ValueTab());
             else if (bits == 32)
                launch_pdl(mx_spmv<float, int32_t>, gq, kRedBlock, nquads, A->sell_ptr.p,
                           A->sell_col.p, A->sell_val32.p, p.p, q.p, S.p, pq, worked, nullptr,
-                          nullptr);
+                          nullptr, ValueTab());
             else if (auni)
                launch_pdl(mx_spmv<__nv_bfloat16, int16_t, true>, gq, kRedBlock, nquads,
                           A->sell_ptr.p, A->sell_d16.p, v16.p, p.p, q.p, S.p, pq, worked, su,
-                          st16);
+                          st16, ValueTab());
             else if (a16)
                launch_pdl(mx_spmv<__nv_bfloat16, int16_t>, gq, kRedBlock, nquads, A->sell_ptr.p,
-                          A->sell_d16.p, v16.p, p.p, q.p, S.p, pq, worked, nullptr, nullptr);
+                          A->sell_d16.p, v16.p, p.p, q.p, S.p, pq, worked, nullptr, nullptr,
+                          ValueTab());
             else
                launch_pdl(mx_spmv<__nv_bfloat16, int32_t>, gq, kRedBlock, nquads, A->sell_ptr.p,
-                          A->sell_col.p, v16.p, p.p, q.p, S.p, pq, worked, nullptr, nullptr);
+                          A->sell_col.p, v16.p, p.p, q.p, S.p, pq, worked, nullptr, nullptr,
+                          ValueTab());
             // algorithmic bytes: value (4 or 2 bytes) and column index (4, 2
             // as a 16-bit offset, or a uniform slice's table) per entry, p
             // gathered, q written, p read for the dot

@@ -78,6 +78,10 @@ constexpr int kHoist = 1;
 // register budget: 65536 / (256 * kQuadBlocks)), and the grid of the
 // kernel chains they are part of.
 constexpr int kQuadBlocks = 8;
+#ifndef KVU
+#define KVU 1
+#endif
+constexpr int kValueUnroll = KVU;
 
 // The four rows r0 .. r0+3 of a uniform slice: w positions, the offset of
 // position k from tp[k].  The values of kHoist positions are loaded before
@@ -113,21 +117,81 @@ __device__ __forceinline__ float4 uniform_quad(const V* __restrict__ vp,
    return acc;
 }
 
+// A slice whose 32 rows also share their values (a constant coefficient on a
+// uniform grid; the learned factor of such a matrix away from the boundary)
+// streams no values at all: ValueTab gives such a slice's entries, (value,
+// offset) per position, all from the caches.
+struct ValueTab {
+   const int2* head;  // per slice: first entry, positions; -1 for other slices
+   const int2* tab;   // FP32 value bits, column - row
+};
+
+// the four rows r0 .. r0+3 of such a slice; products and sums as uniform_quad's
+__device__ __forceinline__ float4 value_quad(const int2* __restrict__ tp, int w,
+                                             const float* __restrict__ x, int r0)
+{
+   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll kValueUnroll
+   for (int k = 0; k < w; ++k) {
+      const int2 e = __ldg(tp + k);
+      const float a = __int_as_float(e.x);
+      const float4 xv = quad_at(x, r0 + e.y);
+      acc.x += a * xv.x;
+      acc.y += a * xv.y;
+      acc.z += a * xv.z;
+      acc.w += a * xv.w;
+   }
+   return acc;
+}
+
+// One warp per slice: the entries of the slices whose rows share offsets
+// (suni[s] >= 0) and values; nnz of those slices added to *count.
+template <class V>
+__global__ void scan_slice_values(int64_t nslices, const int32_t* __restrict__ sp,
+                                  const V* __restrict__ sval, const int32_t* __restrict__ suni,
+                                  const int16_t* __restrict__ stab, int2* head, int2* tab,
+                                  unsigned long long* count)
+{
+   const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+   const int lane = threadIdx.x & 31;
+   if (s >= nslices) return;  // the whole warp shares s
+   const int u = suni[s];
+   const int32_t beg = sp[s];
+   const int w = (sp[s + 1] - beg) >> 5;
+   bool same = u >= 0;
+   for (int k = 0; same && k < w; ++k) {
+      const float v = (float)sval[beg + k * 32 + lane];
+      same = __all_sync(0xffffffffu, __float_as_int(v) ==
+                                        __shfl_sync(0xffffffffu, __float_as_int(v), 0));
+      if (lane == 0) tab[u + k] = make_int2(__float_as_int(v), stab[u + k]);
+   }
+   if (lane == 0) {
+      head[s] = make_int2(same ? u : -1, w);
+      if (same) atomicAdd(count, 32ull * w);
+   }
+}
+
 // y[r0 .. r0+3] = (M x)[r0 .. r0+3] for a SELL-32 matrix M: A itself, or
 // G (lower rows) and G^T (upper rows) of the learned preconditioner, which
 // live on A's slices with BF16 values (the preconditioner's own precision:
 // M = G^T G is still one fixed symmetric positive definite operator).  V is
 // the value type (float or BF16), I the column format (absolute int32 or
-// 16-bit offsets); UNI reads a uniform slice's offsets from its table.
-template <class V, class I, bool UNI>
+// 16-bit offsets); UNI reads a uniform slice's offsets from its table, VAL the values
+// too where they are shared.
+template <class V, class I, bool UNI, bool VAL = false>
 __device__ __forceinline__ float4 sell_quad(const int32_t* __restrict__ sp,
                                             const I* __restrict__ scol,
                                             const V* __restrict__ sval,
                                             const float* __restrict__ x, int64_t r0,
                                             const int32_t* __restrict__ suni,
-                                            const int16_t* __restrict__ stab)
+                                            const int16_t* __restrict__ stab,
+                                            ValueTab vt = ValueTab())
 {
    const int64_t s = r0 >> 5;
+   if (VAL) {
+      const int2 h = __ldg(vt.head + s);
+      if (h.x >= 0) return value_quad(vt.tab + h.x, h.y, x, (int)r0);
+   }
    const int lane0 = (int)(r0 & 31);
    const int32_t beg = sp[s], w = (sp[s + 1] - beg) >> 5;
    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
