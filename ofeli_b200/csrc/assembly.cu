@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) assemble_rows(int64_t nn, const int32_t* 
                                                      const int32_t* __restrict__ emap,
                                                      const int32_t* __restrict__ row_ptr, Elem el,
                                                      double* __restrict__ a, double* __restrict__ b,
-                                                     int* bad)
+                                                     unsigned* bad)
 {
    // each thread sums its row in shared memory (a column per thread)
    __shared__ double racc[kRowAcc * 256];
@@ -48,18 +48,102 @@ __global__ void __launch_bounds__(256) assemble_rows(int64_t nn, const int32_t* 
       const int32_t r = dof[i];   // 1-based equation, 0 for an imposed node
       const double bi =
          gather_node_rows(i, r, n2e_ptr[i], n2e_ptr[i + 1], n2e, elem, emap, row_ptr, el, a,
-                          [&](int64_t e) { atomicMin(bad, (int)e); }, racc + threadIdx.x, 256);
+                          [&](int64_t e) { atomicMin(bad, (unsigned)e); }, racc + threadIdx.x, 256);
       if (r) b[r - 1] = bi;
    }
 }
 
-void check_jacobian(const DBuf<int>& bad)
+// The same over the incidence records of the matrix: what a node needs of an
+// element (number, other nodes, the columns' places in its row) as one
+// 16-byte record (3-D: and a word), the records of 32 nodes side by side, so
+// that a warp streams them in whole lines.  The lists, the connectivity and
+// the element-to-CSR map above are three dependent gathers of 4-byte words
+// (L1 at 50 to 92 % of its rate); here only the other nodes' coordinates and
+// fields are gathered.
+template <class Elem>
+__global__ void __launch_bounds__(256) assemble_incidences(
+   int64_t nn, const int32_t* __restrict__ inc_ptr, const int4* __restrict__ inc,
+   const int32_t* __restrict__ inc_meta, const int32_t* __restrict__ dof,
+   const int32_t* __restrict__ row_ptr, Elem el, double* __restrict__ a, double* __restrict__ b,
+   unsigned* bad)
 {
-   int h = 0;
+   constexpr int NEN = Elem::NEN;
+   __shared__ double racc_all[kRowAcc * 256];
+   double* racc = racc_all + threadIdx.x;  // entry j at racc[256 j]
+   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += stride) {
+      const int64_t s = i >> 5;
+      const int32_t beg = inc_ptr[s], w = inc_ptr[s + 1] - beg;
+      const int64_t at = (int64_t)beg * 32 + (i & 31);
+      const int32_t r = dof[i];   // 1-based equation, 0 for an imposed node
+      int32_t rs = 0, rl = 0;
+      if (r) {
+         rs = row_ptr[r - 1];
+         rl = row_ptr[r] - rs;
+         for (int32_t j = 0; j < rl; ++j) racc[j * 256] = 0.0;
+      }
+      Corners<NEN, Elem::DIM> own;
+      own.load(0, el.coords(), i);
+      double bi = 0.0;
+      int4 next = w > 0 ? inc[at] : make_int4(-1, 0, 0, 0);
+      int32_t next_meta = NEN == 4 && w > 0 ? inc_meta[at] : 0;
+      for (int32_t p = 0; p < w; ++p) {
+         const int4 rec = next;
+         const int32_t meta = NEN == 3 ? rec.w : next_meta;
+         if (p + 1 < w) {
+            next = inc[at + (int64_t)(p + 1) * 32];
+            if (NEN == 4) next_meta = inc_meta[at + (int64_t)(p + 1) * 32];
+         }
+         if (rec.x < 0) break;   // the node's last element was the one before
+         const int li = meta & 3;
+         // the element's nodes in its own order: the node itself at place li
+         const int32_t other[3] = {rec.y, rec.z, rec.w};
+         int32_t en[NEN];
+         Corners<NEN, Elem::DIM> X, O;
+#pragma unroll
+         for (int k = 0; k < NEN - 1; ++k) O.load(k, el.coords(), other[k]);
+#pragma unroll
+         for (int j = 0; j < NEN; ++j) {
+            const int hi = j < NEN - 1 ? j : NEN - 2, lo = j > 0 ? j - 1 : 0;
+            en[j] = j == li ? (int32_t)i : j < li ? other[hi] : other[lo];
+#pragma unroll
+            for (int d = 0; d < Elem::DIM; ++d)
+               X.x[j][d] = j == li ? own.x[0][d] : j < li ? O.x[hi][d] : O.x[lo][d];
+         }
+         if (!r) {   // no row here: only the Jacobian check of the elements it leads
+            if (li == 0 && !el.geometry_ok(X)) atomicMin(bad, (unsigned)rec.x);
+            continue;
+         }
+         int32_t off[NEN];
+#pragma unroll
+         for (int j = 0; j < NEN; ++j) {
+            off[j] = inc_offset(meta, j);
+            if (off[j] == kIncNone) off[j] = -1;
+         }
+         double krow[NEN], frow;
+         if (!el.row(rec.x, X, en, li, i, off, krow, frow)) {
+            if (li == 0) atomicMin(bad, (unsigned)rec.x);
+            continue;
+         }
+#pragma unroll
+         for (int j = 0; j < NEN; ++j)
+            if (off[j] >= 0) racc[off[j] * 256] += krow[j];
+         bi += frow;
+      }
+      if (r) {
+         for (int32_t j = 0; j < rl; ++j) a[rs + j] = racc[j * 256];
+         b[r - 1] = bi;
+      }
+   }
+}
+
+void check_jacobian(const DBuf<unsigned>& bad)
+{
+   unsigned h = 0;
    bad.download(&h, 1);
-   if (h != INT32_MAX)
+   if (h != 0xffffffffu)
       throw Error(OFG_ERR_JACOBIAN,
-                  "non-positive Jacobian determinant in element " + std::to_string(h + 1));
+                  "non-positive Jacobian determinant in element " + std::to_string((int64_t)h + 1));
 }
 
 // Launches the row-gather kernel for one element kind and checks Jacobians.
@@ -68,9 +152,8 @@ void assemble(ofg_mesh* m, ofg_matrix* A, const Elem& el, double* db, int node_f
               int elem_fields)
 {
    OFG_REQUIRE(A->mesh == m, OFG_ERR_ARG, "matrix pattern was not built from this mesh");
-   DBuf<int> bad(1);
-   int big = INT32_MAX;
-   bad.upload(&big, 1);
+   DBuf<unsigned> bad(1);   // lowest bad element; all ones: none
+   OFG_CUDA(cudaMemsetAsync(bad.p, 0xFF, sizeof(unsigned), stream()));
    if (m->nn) {
       const int nen = m->nen;
       double bytes = 4.0 * (m->nn + 1) + 8.0 * nen * m->ne + 8.0 * m->dim * m->nn + 8.0 * m->nn +
@@ -79,9 +162,15 @@ void assemble(ofg_mesh* m, ofg_matrix* A, const Elem& el, double* db, int node_f
                      8.0 * A->nnz + 8.0 * A->n;
       int* worked = prof_begin();
       if (worked) OFG_CUDA(cudaMemsetAsync(worked, 1, sizeof(int), stream()));
-      assemble_rows<Elem><<<grid_for(m->nn, 256, 16), 256, 0, stream()>>>(
-          m->nn, m->n2e_ptr.p, m->n2e.p, m->elem.p, m->dof.p, A->emap.p, A->row_ptr.p, el,
-          A->val.p, db, bad.p);
+      const unsigned grid = grid_for(m->nn, 256, 16);
+      if (A->inc_on)
+         assemble_incidences<Elem><<<grid, 256, 0, stream()>>>(
+            m->nn, A->inc_ptr.p, A->inc.p, A->inc_meta.p, m->dof.p, A->row_ptr.p, el, A->val.p, db,
+            bad.p);
+      else
+         assemble_rows<Elem><<<grid, 256, 0, stream()>>>(
+            m->nn, m->n2e_ptr.p, m->n2e.p, m->elem.p, m->dof.p, A->emap.p, A->row_ptr.p, el,
+            A->val.p, db, bad.p);
       prof_end(PROF_ASSEMBLY, bytes);
       count_launch();
       OFG_LAUNCH_CHECK();

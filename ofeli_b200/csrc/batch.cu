@@ -925,6 +925,7 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
             gather(B->dof, P.node_off, m->dof.p, m->nn);
             gather(B->n2e_ptr, P.n2p_off, m->n2e_ptr.p, m->nn + 1);
             gather(B->n2e, P.n2e_off, m->n2e.p, m->ne * nen);
+            ensure_emap(A);
             gather(B->emap, P.elem_off * nen * nen, A->emap.p, m->ne * nen * nen);
             gather(B->row_ptr, P.rp_off, A->row_ptr.p, A->n + 1);
             gather(B->col, P.nnz_off, A->col.p, A->nnz);

@@ -16,32 +16,100 @@ __device__ __forceinline__ double dot3(const double* a, const double* b)
    return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 
-// Triang3::set (src/shape_functions/Triang3.cpp:68-93)
-__device__ __forceinline__ bool tri3(const double* xy, const int32_t* en, double g[3][3],
-                                     double& area)
+// Six quotients by one divisor, correctly rounded as six divisions would be,
+// from one reciprocal: with r = RN(1/d), q = RN(a r) is off by at most two
+// units in the last place, one step q + r (a - q d), its residual exact in a
+// fused multiply-add, leaves it off by less than one, and by Markstein's
+// theorem (IBM J. Res. Dev. 34(1), 1990) the second step rounds correctly,
+// barring overflow and underflow: `plain` says whether all exponents are far
+// from both (else divide).  A division is some 25 instructions, and the six
+// of an element were a third of the assembly's.
+__device__ __forceinline__ bool plain_exponent(double v)
 {
-   double x0 = xy[2 * en[0]], y0 = xy[2 * en[0] + 1];
-   double x1 = xy[2 * en[1]], y1 = xy[2 * en[1] + 1];
-   double x2 = xy[2 * en[2]], y2 = xy[2 * en[2] + 1];
+   // 2^-500 <= |v| < 2^501, or 0
+   return ((__double2hiint(v) & 0x7ff00000u) - (523u << 20) <= (1000u << 20)) || v == 0.0;
+}
+__device__ __forceinline__ double quotient(double a, double d, double r)
+{
+   double q = __dmul_rn(a, r);
+   q = __fma_rn(__fma_rn(-q, d, a), r, q);
+   return __fma_rn(__fma_rn(-q, d, a), r, q);
+}
+
+// An element's node coordinates: held in registers (Corners), or read from
+// the mesh where they are used (CornersAt; the batched solver's kernel, whose
+// registers are capped, is 3 % slower with the other, and keeps the
+// divisions, too).
+template <int NEN, int DIM>
+struct Corners {
+   static constexpr bool kQuotients = true;
+   double x[NEN][DIM];
+   __device__ __forceinline__ double operator()(int k, int d) const { return x[k][d]; }
+   __device__ __forceinline__ void load(int k, const double* xyz, int64_t node)
+   {
+      if (DIM == 2) {
+         // (coordinate pairs of a mesh are 16-byte aligned)
+         const double2 p = *reinterpret_cast<const double2*>(xyz + 2 * node);
+         x[k][0] = p.x;
+         x[k][1] = p.y;
+      }
+      else {
+#pragma unroll
+         for (int d = 0; d < DIM; ++d) x[k][d] = xyz[DIM * node + d];
+      }
+   }
+};
+template <int NEN, int DIM>
+struct CornersAt {
+   static constexpr bool kQuotients = false;
+   const double* xyz;
+   const int32_t (&en)[NEN];
+   __device__ __forceinline__ double operator()(int k, int d) const { return xyz[DIM * en[k] + d]; }
+};
+
+// Triang3::set (src/shape_functions/Triang3.cpp:68-93)
+template <class Geometry>
+__device__ __forceinline__ bool tri3(const Geometry& X, double g[3][3], double& area)
+{
+   double x0 = X(0, 0), y0 = X(0, 1);
+   double x1 = X(1, 0), y1 = X(1, 1);
+   double x2 = X(2, 0), y2 = X(2, 1);
    double det = (x1 - x0) * (y2 - y0) - (y1 - y0) * (x2 - x0);
    area = 0.5 * det;
    if (!(det > 0.0)) return false;
-   g[0][0] = (y1 - y2) / det; g[0][1] = (x2 - x1) / det; g[0][2] = 0.0;
-   g[1][0] = (y2 - y0) / det; g[1][1] = (x0 - x2) / det; g[1][2] = 0.0;
-   g[2][0] = (y0 - y1) / det; g[2][1] = (x1 - x0) / det; g[2][2] = 0.0;
+   if constexpr (!Geometry::kQuotients) {
+      g[0][0] = (y1 - y2) / det; g[0][1] = (x2 - x1) / det; g[0][2] = 0.0;
+      g[1][0] = (y2 - y0) / det; g[1][1] = (x0 - x2) / det; g[1][2] = 0.0;
+      g[2][0] = (y0 - y1) / det; g[2][1] = (x1 - x0) / det; g[2][2] = 0.0;
+      return true;
+   }
+   const double n[6] = {y1 - y2, x2 - x1, y2 - y0, x0 - x2, y0 - y1, x1 - x0};
+   bool plain = plain_exponent(det);
+#pragma unroll
+   for (int k = 0; k < 6; ++k) plain = plain && plain_exponent(n[k]);
+   if (plain) {
+      const double r = 1.0 / det;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) g[k >> 1][k & 1] = quotient(n[k], det, r);
+   }
+   else {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) g[k >> 1][k & 1] = n[k] / det;
+   }
+   g[0][2] = g[1][2] = g[2][2] = 0.0;
    return true;
 }
 
 // Tetra4::CalculateShape (src/shape_functions/Tetra4.cpp:76-114): Jacobian,
 // its cofactors, det, gradients J^{-T} grad(phi_ref); volume det/6.
-__device__ __forceinline__ bool tet4(const double* xyz, const int32_t* en, double g[4][3],
-                                     double& vol)
+template <class Geometry>
+__device__ __forceinline__ bool tet4(const Geometry& G, double g[4][3], double& vol)
 {
    double X[4][3];
 #pragma unroll
    for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) X[k][d] = xyz[3 * en[k] + d];
+      for (int d = 0; d < 3; ++d) X[k][d] = G(k, d);
    // J(r,c) = sum_k dphi_k/dxi_c * x_k[r]; reference gradients (-1,-1,-1), e1, e2, e3
    double J[3][3];
 #pragma unroll
@@ -102,22 +170,26 @@ __device__ __forceinline__ void gradient_of(const double (&g)[NEN][3], int li, d
 // (src/equations/laplace/Laplace2DT3.cpp:131-143)
 struct LaplaceT3 {
    static constexpr int NEN = 3;
+   static constexpr int DIM = 2;
    const double* xy;
+   __device__ __forceinline__ const double* coords() const { return xy; }
    const int32_t* code;
    const double* kel;
    const double* f;
    const double* bc;
-   __device__ __forceinline__ bool geometry_ok(const int32_t (&en)[3]) const
+   template <class Geometry>
+   __device__ __forceinline__ bool geometry_ok(const Geometry& X) const
    {
       double g[3][3], area;
-      return tri3(xy, en, g, area);
+      return tri3(X, g, area);
    }
-   __device__ __forceinline__ bool row(int64_t e, const int32_t (&en)[3], int li, int64_t node,
+   template <class Geometry>
+   __device__ __forceinline__ bool row(int64_t e, const Geometry& X, const int32_t (&en)[3], int li, int64_t node,
                                        const int32_t (&pos)[3], double (&krow)[3],
                                        double& frow) const
    {
       double g[3][3], area, gl[3];
-      if (!tri3(xy, en, g, area)) return false;
+      if (!tri3(X, g, area)) return false;
       gradient_of<3>(g, li, gl);
       const double k = kel ? kel[e] : 1.0;
 #pragma unroll
@@ -132,22 +204,26 @@ struct LaplaceT3 {
 // (src/equations/therm/DC3DT4.cpp:128-135, 207-211)
 struct DiffusionT4 {
    static constexpr int NEN = 4;
+   static constexpr int DIM = 3;
    const double* xyz;
+   __device__ __forceinline__ const double* coords() const { return xyz; }
    const int32_t* code;
    const double* kel;
    const double* f;
    const double* bc;
-   __device__ __forceinline__ bool geometry_ok(const int32_t (&en)[4]) const
+   template <class Geometry>
+   __device__ __forceinline__ bool geometry_ok(const Geometry& X) const
    {
       double g[4][3], vol;
-      return tet4(xyz, en, g, vol);
+      return tet4(X, g, vol);
    }
-   __device__ __forceinline__ bool row(int64_t e, const int32_t (&en)[4], int li, int64_t node,
+   template <class Geometry>
+   __device__ __forceinline__ bool row(int64_t e, const Geometry& X, const int32_t (&en)[4], int li, int64_t node,
                                        const int32_t (&pos)[4], double (&krow)[4],
                                        double& frow) const
    {
       double g[4][3], vol, gl[3];
-      if (!tet4(xyz, en, g, vol)) return false;
+      if (!tet4(X, g, vol)) return false;
       gradient_of<4>(g, li, gl);
       const double c = (kel ? kel[e] : 1.0) * vol;
 #pragma unroll
@@ -168,24 +244,28 @@ struct DiffusionT4 {
 // after updateBC has lifted the imposed values with eMat.
 struct ConvDiffT3 {
    static constexpr int NEN = 3;
+   static constexpr int DIM = 2;
    const double* xy;
+   __device__ __forceinline__ const double* coords() const { return xy; }
    const int32_t* code;
    double eps, dti;
    const double* v;
    const double* u_old;
    const double* bc;
    int scheme;
-   __device__ __forceinline__ bool geometry_ok(const int32_t (&en)[3]) const
+   template <class Geometry>
+   __device__ __forceinline__ bool geometry_ok(const Geometry& X) const
    {
       double g[3][3], area;
-      return tri3(xy, en, g, area);
+      return tri3(X, g, area);
    }
-   __device__ __forceinline__ bool row(int64_t, const int32_t (&en)[3], int li, int64_t,
+   template <class Geometry>
+   __device__ __forceinline__ bool row(int64_t, const Geometry& X, const int32_t (&en)[3], int li, int64_t,
                                        const int32_t (&pos)[3], double (&krow)[3],
                                        double& frow) const
    {
       double g[3][3], area, gl[3];
-      if (!tri3(xy, en, g, area)) return false;
+      if (!tri3(X, g, area)) return false;
       gradient_of<3>(g, li, gl);
       const double cc = kSixth * area, dd = 0.5 * cc, cl = kThird * area;
       const double v3[3] = {v[2 * en[0]] + v[2 * en[1]] + v[2 * en[2]],
@@ -219,9 +299,6 @@ struct ConvDiffT3 {
 // report(e).  Used by the single-problem kernel (assembly.cu) and the
 // batched solver (batch.cu).  The connectivity of the next element is loaded
 // while the current one is computed.
-// longest row summed in shared memory by gather_node_rows
-constexpr int kRowAcc = 16;
-
 template <class Elem, class Report>
 __device__ __forceinline__ double gather_node_rows(int64_t i, int32_t r, int32_t q0, int32_t q1,
                                                    const int32_t* __restrict__ n2e,
@@ -267,7 +344,7 @@ __device__ __forceinline__ double gather_node_rows(int64_t i, int32_t r, int32_t
       for (int j = NEN - 1; j > 0; --j)
          if (en[j] == (int32_t)i) li = j;
       if (!r) {   // no row here: only the Jacobian check of the elements it leads
-         if (li == 0 && !el.geometry_ok(en)) report(e);
+         if (li == 0 && !el.geometry_ok(CornersAt<NEN, Elem::DIM>{el.coords(), en})) report(e);
          continue;
       }
       int32_t pos[NEN];
@@ -275,7 +352,7 @@ __device__ __forceinline__ double gather_node_rows(int64_t i, int32_t r, int32_t
 #pragma unroll
       for (int j = 0; j < NEN; ++j) pos[j] = mp[j];
       double krow[NEN], frow;
-      if (!el.row(e, en, li, i, pos, krow, frow)) {
+      if (!el.row(e, CornersAt<NEN, Elem::DIM>{el.coords(), en}, en, li, i, pos, krow, frow)) {
          if (li == 0) report(e);
          continue;
       }

@@ -59,8 +59,8 @@ struct FGState {
    int stop;           // the cycle is over
    int done;           // FP64 true residual <= toler
    int skip_end;       // the cycle-end kernels of this batch do nothing
-   int zero_diag;      // a diagonal entry is zero (FP32 values: checked with the first state read)
-   int pad;
+   int zero_diag;      // a diagonal entry is zero (checked with the first state read)
+   int inexact;        // a value of A is not exact in BF16 (likewise)
 };
 
 // r = b - q (FP64); ||r||, ||b|| (first call); the FP64 convergence test
@@ -567,9 +567,17 @@ void fgmres_mixed(ofg_prec* P, int inner_bits, const double* b, double* x, int m
                "inner_bits must be 32, 16 or 0 (automatic)");
    OFG_REQUIRE(inner_tol > 0 && inner_tol < 1, OFG_ERR_ARG, "inner_tol must be in (0, 1)");
    const int64_t n = A->n;
-   // FP32 values asked for: both SELL copies of new values in one pass
+   DBuf<FGState> S(1);
+   S.zero();
+   // new values go into the SELL copies in one pass: FP64 and FP32, and, for
+   // the automatic format, BF16 with its exactness flag
+   DBuf<__nv_bfloat16> v16;
+   const __nv_bfloat16* vals16 = nullptr;
    if (inner_bits == 32) ensure_sell32(A);
-   else ensure_sell(A);
+   else {
+      if (inner_bits == 0) vals16 = refresh_sell_all(A, &S.p->inexact);
+      ensure_sell(A);
+   }
    ensure_dpos(A);
    OFG_REQUIRE(A->dpos_complete, OFG_ERR_PIVOT, "a row has no diagonal entry");
    bool learned = P->type == OFG_LEARNED;
@@ -587,49 +595,29 @@ void fgmres_mixed(ofg_prec* P, int inner_bits, const double* b, double* x, int m
    a.d16 = ensure_sell_d16(A);
    if (a.d16) ensure_sell_uniform(A);
    a.uni = a.d16 && mostly_uniform(A);
-   // bad[0]: zero diagonal entry; bad[1]: a value of A is not exact in BF16
-   DBuf<int> bad(2);
-   bad.zero();
-   DBuf<__nv_bfloat16> v16;
-   if (inner_bits != 32) {
+   if (inner_bits != 32 && !vals16) {
       v16.alloc(A->sell_val.n);
       fg_cast_bf16<<<grid_for(A->sell_val.n, 256), 256, 0, stream()>>>(A->sell_val.n,
                                                                        A->sell_val.p, v16.p,
-                                                                       bad.p + 1);
+                                                                       &S.p->inexact);
       count_launch();
+      vals16 = v16.p;
    }
-   DBuf<FGState> S(1);
-   S.zero();
    DBuf<float> dinv(nv);
-   // with FP32 values nothing waits for the zero-diagonal flag: it travels
-   // in the solver state and is checked at its first read
+   // nothing waits for the zero-diagonal and exactness flags: they travel in
+   // the solver state and are checked at its first read
    fg_inv_diag<<<grid_for(nv, 256), 256, 0, stream()>>>(n, npad, A->dpos.p, A->val.p, dinv.p,
                                                          P->type == OFG_IDENT ? 1 : 0,
-                                                         inner_bits == 32 ? &S.p->zero_diag : bad.p);
+                                                         &S.p->zero_diag);
    count_launch();
    OFG_LAUNCH_CHECK();
-   int hb[2] = {0, 0};
-   if (inner_bits != 32) {
-      bad.download(hb, 2);
-      OFG_REQUIRE(!hb[0], OFG_ERR_PIVOT, "zero diagonal entry");
-   }
-   // automatic format: BF16 values only when every value is exact in BF16
-   const bool use16 = inner_bits == 16 || (inner_bits == 0 && !hb[1]);
-   if (use16) {
-      a.bf16 = true;
-      a.val = v16.p;
-   }
-   else {
-      v16.release();
-      ensure_sell32(A);
-      a.val = A->sell_val32.p;
-   }
-   a.bytes = (use16 ? 2.0 : 4.0) * A->nnz + index_bytes(A, a.d16, a.uni);
-
    const int64_t ldz = nv + 8;  // Z vectors are gathered: 8 elements of slack
    DBuf<double> V((size_t)(m + 1) * nv), w(nv), r(n > 0 ? n : 1), q64(n > 0 ? n : 1);
    DBuf<float> Z((size_t)m * ldz), w32(nv), v32(learned ? ldz : 1), t32(learned ? ldz : 1);
-   Z.zero();
+   // (the slack: loaded, never used; the rows are written before they are read)
+   if (m > 0)
+      OFG_CUDA(cudaMemset2DAsync(Z.p + nv, ldz * sizeof(float), 0, (ldz - nv) * sizeof(float), m,
+                                 stream()));
    v32.zero();
    t32.zero();
    DBuf<double> H((size_t)(m + 1) * (m + 1)), s(m + 1), cs(m + 1), sn(m + 1), y(m + 1), h2(m + 1);
@@ -663,6 +651,18 @@ void fgmres_mixed(ofg_prec* P, int inner_bits, const double* b, double* x, int m
    true_residual(1);
    S.download(&h, 1);
    OFG_REQUIRE(!h.zero_diag, OFG_ERR_PIVOT, "zero diagonal entry");
+   // automatic format: BF16 values only when every value is exact in BF16
+   const bool use16 = inner_bits == 16 || (inner_bits == 0 && !h.inexact);
+   if (use16) {
+      a.bf16 = true;
+      a.val = vals16;
+   }
+   else {
+      v16.release();
+      ensure_sell32(A);
+      a.val = A->sell_val32.p;
+   }
+   a.bytes = (use16 ? 2.0 : 4.0) * A->nnz + index_bytes(A, a.d16, a.uni);
    int n_outer = 0, n_inner = 0, no_gain = 0;
    double last_rel = h.rel;
    while (!h.done && n_outer < max_outer && n_inner < max_inner && n > 0) {

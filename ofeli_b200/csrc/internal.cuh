@@ -2,6 +2,8 @@
 // translation units share.
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 // Device CSR matrix.  The CSR arrays are the master copy (OFELI's SpMatrix
@@ -55,7 +57,14 @@ struct ofg_matrix {
 
    // element-to-CSR map of the mesh this pattern came from
    ofg_mesh* mesh = nullptr;
+   // (built on first use: the batched solver, rows longer than kRowAcc)
    ofg::DBuf<int32_t> emap;  // ne * nen * nen, -1 where a DOF is imposed
+   // the assembly's incidence records (see assembly.cu): node slices of 32,
+   // record p of lane l of slice s at (inc_ptr[s] + p) * 32 + l
+   bool inc_on = false;
+   ofg::DBuf<int32_t> inc_ptr;   // slices + 1
+   ofg::DBuf<int4> inc;          // element (-1: none), its other nodes (3-D: three)
+   ofg::DBuf<int32_t> inc_meta;  // own place in the element, row offsets of its columns
 };
 
 struct ofg_mesh {
@@ -164,6 +173,10 @@ void ensure_dpos(ofg_matrix* A);
 void ensure_sell(ofg_matrix* A);
 void ensure_sell32(ofg_matrix* A);
 void ensure_sell_bf16(ofg_matrix* A);
+// new values into the FP64, FP32 and BF16 SELL copies in one pass, *inexact
+// set when one is not exact in BF16; the BF16 copy, or null, with nothing
+// done, when the copies are not stale or not laid out yet
+const __nv_bfloat16* refresh_sell_all(ofg_matrix* A, int* inexact);
 // builds the 16-bit column offsets once per pattern; true when they fit
 bool ensure_sell_d16(ofg_matrix* A);
 // after ensure_sell_d16 returned true
@@ -177,6 +190,14 @@ void matrix_finish_pattern(ofg_matrix* A);
 // once those hold the mesh (mesh.cu)
 ofg_mesh* new_mesh(int dim, int64_t nn, int64_t ne);
 void finish_mesh(ofg_mesh* m);
+// the element-to-CSR map of a matrix made from a mesh
+void ensure_emap(ofg_matrix* A);
+// longest row the assembly sums in shared memory
+constexpr int kRowAcc = 16;
+// an incidence record's meta word: bits 0-1 the node's place in the element,
+// then 5 bits per element node: its column's offset in the row, or kIncNone
+constexpr int kIncNone = 31;
+__host__ __device__ inline int inc_offset(int32_t meta, int j) { return (meta >> (2 + 5 * j)) & 31; }
 void scan_exclusive_i64(const int64_t* d_in, int64_t* d_out, int64_t n);
 
 // prec.cu

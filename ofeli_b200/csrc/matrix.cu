@@ -167,6 +167,25 @@ __global__ void sell_values_both(int64_t total, const int32_t* ssrc, const doubl
    }
 }
 
+// and the BF16 one, *inexact = 1 when some value is not exact in BF16 (a NaN
+// never is)
+__global__ void sell_values_all(int64_t total, const int32_t* ssrc, const double* val, double* sval,
+                                float* sval32, __nv_bfloat16* sval16, int* inexact)
+{
+   int64_t stride = (int64_t)gridDim.x * blockDim.x;
+   int lost = 0;
+   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+      const int32_t s = ssrc[i];
+      const double v = s >= 0 ? val[s] : 0.0;
+      const __nv_bfloat16 h = (__nv_bfloat16)v;
+      sval[i] = v;
+      sval32[i] = (float)v;
+      sval16[i] = h;
+      lost |= (double)__bfloat162float(h) != v;
+   }
+   if (__syncthreads_or(lost) && threadIdx.x == 0) atomicOr(inexact, 1);
+}
+
 __global__ void sell_values_bf16(int64_t total, const int32_t* ssrc, const double* val,
                                  uint16_t* sval)
 {
@@ -522,6 +541,25 @@ void ensure_sell32(ofg_matrix* A)
       OFG_LAUNCH_CHECK();
       A->sell32_version = A->version;
    }
+}
+
+const __nv_bfloat16* refresh_sell_all(ofg_matrix* A, int* inexact)
+{
+   if (!A->sell_ready || A->sell_version == A->version) return nullptr;
+   const int64_t total = A->sell_val.n;
+   A->sell_val32.reserve(total);
+   // (kept with the matrix: a buffer that comes and goes with every call
+   // splits the pool's free blocks, and the call's large vectors then have to
+   // be mapped anew, 500 us at 1025^2)
+   A->sell_valbf.reserve(total);
+   auto* v16 = reinterpret_cast<__nv_bfloat16*>(A->sell_valbf.p);
+   sell_values_all<<<grid_for(total, 256), 256, 0, stream()>>>(
+      total, A->sell_src.p, A->val.p, A->sell_val.p, A->sell_val32.p, v16, inexact);
+   count_launch();
+   OFG_LAUNCH_CHECK();
+   A->sell_version = A->sell32_version = A->version;
+   A->sellbf_version = 0;  // (ensure_sell_bf16 rounds by way of FP32)
+   return v16;
 }
 
 void ensure_sell_bf16(ofg_matrix* A)

@@ -227,7 +227,141 @@ __global__ void build_emap(int64_t ne, int nen, const int32_t* elem, const int32
    }
 }
 
+__device__ __forceinline__ int32_t find_column(const int32_t* row_ptr, const int32_t* col, int32_t r,
+                                               int32_t c)
+{
+   int32_t lo = row_ptr[r - 1], hi = row_ptr[r] - 1;
+   while (lo <= hi) {
+      const int32_t mid = (lo + hi) >> 1, v = col[mid];
+      if (v == c - 1) return mid;
+      if (v < c - 1) lo = mid + 1;
+      else hi = mid - 1;
+   }
+   return -1;
+}
+
+// most elements around a node of each slice of 32 nodes
+__global__ void inc_widths(int64_t nn, int64_t nslices, const int32_t* n2e_ptr, int64_t* width)
+{
+   const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+   if (s >= nslices) return;  // the whole warp shares s
+   const int64_t i = s * 32 + (threadIdx.x & 31);
+   int w = i < nn ? n2e_ptr[i + 1] - n2e_ptr[i] : 0;
+   w = __reduce_max_sync(0xffffffffu, w);
+   if ((threadIdx.x & 31) == 0) width[s] = w;
+}
+
+// the incidence records of every node, its elements ascending
+template <int NEN>
+__global__ void inc_fill(int64_t nn, int64_t nslices, const int64_t* start, const int32_t* n2e_ptr,
+                         const int32_t* n2e, const int32_t* elem, const int32_t* dof,
+                         const int32_t* row_ptr, const int32_t* col, int32_t* inc_ptr, int4* inc,
+                         int32_t* inc_meta, int* missing)
+{
+   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+   const int64_t s = t >> 5;
+   if (s >= nslices) return;
+   const int lane = (int)(t & 31);
+   const int64_t i = t;
+   const int64_t beg = start[s];
+   const int w = (int)(start[s + 1] - beg);
+   if (lane == 0) {
+      inc_ptr[s] = (int32_t)beg;
+      if (s == nslices - 1) inc_ptr[nslices] = (int32_t)start[nslices];
+   }
+   const int32_t q0 = i < nn ? n2e_ptr[i] : 0, deg = i < nn ? n2e_ptr[i + 1] - q0 : 0;
+   const int32_t r = i < nn ? dof[i] : 0;
+   for (int p = 0; p < w; ++p) {
+      int4 rec = make_int4(-1, 0, 0, 0);
+      int32_t meta = 0;
+      if (p < deg) {
+         const int32_t e = n2e[q0 + p];
+         int32_t en[NEN], other[3] = {0, 0, 0};
+         int li = 0, k = 0;
+         for (int j = 0; j < NEN; ++j) en[j] = elem[(int64_t)NEN * e + j];
+         for (int j = NEN - 1; j > 0; --j)
+            if (en[j] == (int32_t)i) li = j;
+         for (int j = 0; j < NEN; ++j)
+            if (j != li) other[k++] = en[j];
+         meta = li;
+         for (int j = 0; j < NEN; ++j) {
+            int off = kIncNone;
+            const int32_t c = dof[en[j]];
+            if (r && c) {
+               const int32_t pos = find_column(row_ptr, col, r, c);
+               if (pos < 0) atomicOr(missing, 1);
+               else off = pos - row_ptr[r - 1];
+            }
+            meta |= off << (2 + 5 * j);
+         }
+         rec = make_int4(e, other[0], other[1], NEN == 3 ? meta : other[2]);
+      }
+      const int64_t at = (beg + p) * 32 + lane;
+      inc[at] = rec;
+      if (NEN == 4) inc_meta[at] = meta;
+   }
+}
+
 }  // namespace
+
+void ensure_emap(ofg_matrix* A)
+{
+   if (A->emap.p) return;
+   const ofg_mesh* m = A->mesh;
+   const int64_t nmap = m->ne * m->nen * m->nen;
+   A->emap.alloc(nmap > 0 ? nmap : 1);
+   DBuf<int> missing(1);
+   missing.zero();
+   if (nmap) {
+      build_emap<<<grid_for(nmap, 256), 256, 0, stream()>>>(m->ne, m->nen, m->elem.p, m->dof.p,
+                                                             A->row_ptr.p, A->col.p, A->emap.p,
+                                                             missing.p);
+      count_launch();
+      OFG_LAUNCH_CHECK();
+   }
+   int h = 0;
+   missing.download(&h, 1);
+   OFG_REQUIRE(!h, OFG_ERR_PATTERN, "scatter map found a pair outside the pattern");
+}
+
+// The incidence records, when every row fits the assembly's row sums
+static void build_incidences(ofg_matrix* A)
+{
+   const ofg_mesh* m = A->mesh;
+   const int64_t ns = (m->nn + 31) / 32;
+   if (A->max_row > kRowAcc || ns == 0) return;
+   DBuf<int64_t> w(ns + 1), start(ns + 1);
+   w.zero();
+   inc_widths<<<(unsigned)((ns * 32 + 255) / 256), 256, 0, stream()>>>(m->nn, ns, m->n2e_ptr.p, w.p);
+   count_launch();
+   OFG_LAUNCH_CHECK();
+   scan_exclusive_i64(w.p, start.p, ns + 1);
+   int64_t total = 0;
+   OFG_CUDA(cudaMemcpyAsync(&total, start.p + ns, 8, cudaMemcpyDeviceToHost, stream()));
+   OFG_CUDA(cudaStreamSynchronize(stream()));
+   // a few nodes with very many elements would blow the slices up
+   if (total > INT32_MAX || total * 32 > 4 * m->ne * m->nen + 4096) return;
+   A->inc_ptr.alloc(ns + 1);
+   A->inc.alloc(total > 0 ? total * 32 : 1);
+   A->inc_meta.alloc(m->nen == 4 && total > 0 ? total * 32 : 1);
+   DBuf<int> missing(1);
+   missing.zero();
+   const unsigned grid = (unsigned)((ns * 32 + 127) / 128);
+   if (m->nen == 3)
+      inc_fill<3><<<grid, 128, 0, stream()>>>(m->nn, ns, start.p, m->n2e_ptr.p, m->n2e.p, m->elem.p,
+                                              m->dof.p, A->row_ptr.p, A->col.p, A->inc_ptr.p,
+                                              A->inc.p, A->inc_meta.p, missing.p);
+   else
+      inc_fill<4><<<grid, 128, 0, stream()>>>(m->nn, ns, start.p, m->n2e_ptr.p, m->n2e.p, m->elem.p,
+                                              m->dof.p, A->row_ptr.p, A->col.p, A->inc_ptr.p,
+                                              A->inc.p, A->inc_meta.p, missing.p);
+   count_launch();
+   OFG_LAUNCH_CHECK();
+   int h = 0;
+   missing.download(&h, 1);
+   OFG_REQUIRE(!h, OFG_ERR_PATTERN, "scatter map found a pair outside the pattern");
+   A->inc_on = true;
+}
 
 // Equation numbers, node-to-element lists (see internal.cuh).
 void finish_mesh(ofg_mesh* m)
@@ -475,23 +609,12 @@ int ofg_matrix_create_from_mesh(ofg_mesh* m, ofg_matrix** out)
             A->col.p, 1, overflow.p);
          count_launch();
          OFG_LAUNCH_CHECK();
-         // element -> CSR scatter map
-         int64_t nmap = m->ne * m->nen * m->nen;
-         A->emap.alloc(nmap > 0 ? nmap : 1);
-         DBuf<int> missing(1);
-         missing.zero();
-         if (nmap) {
-            build_emap<<<grid_for(nmap, 256), 256, 0, stream()>>>(m->ne, m->nen, m->elem.p,
-                                                                   m->dof.p, A->row_ptr.p, A->col.p,
-                                                                   A->emap.p, missing.p);
-            count_launch();
-            OFG_LAUNCH_CHECK();
-         }
-         int h = 0;
-         missing.download(&h, 1);
-         OFG_REQUIRE(!h, OFG_ERR_PATTERN, "scatter map found a pair outside the pattern");
          A->mesh = m;
          matrix_finish_pattern(A);
+         // what the assembly walks: the incidence records, or the element ->
+         // CSR scatter map
+         build_incidences(A);
+         if (!A->inc_on) ensure_emap(A);
       }
       catch (...) {
          delete A;
