@@ -122,6 +122,7 @@ struct WavePlan {
    int64_t tiles = 0;         // 32-step layout tiles
    DBuf<int32_t> line, shift, dshift, eoff;
    DBuf<int32_t> g_line, g_tile, g_nch, g_edge, g_sm1, tile_g;
+   DBuf<int32_t> stpos;       // forward, D-ILU: transposed positions in SELL order
    DBuf<double> coef, ecoef;  // step order; ecoef: natural order
    DBuf<double> edge;         // last lines of the groups on their way to the next group
    DBuf<double> gdot;
@@ -221,6 +222,7 @@ void fill_sentinel(double* p, int64_t n);
 // row rho - 1, logical order; tpos: transposed positions when a
 // factorisation is wanted); false when the matrix has no such lines
 bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpos, WavePlan& p);
+void wave_diagonal(ofg_prec* P, int invert, int* bad);  // P->pivot from the current diagonal
 void wave_factor(ofg_prec* P);                // D-ILU pivots of the current values
 void wave_values(ofg_prec* P, WavePlan& p);   // the plan's copy of values and pivots
 void wave_solve(ofg_prec* P, bool fwd, const double* in, double* out, double* reset,

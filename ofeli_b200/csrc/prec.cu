@@ -1174,7 +1174,8 @@ void prec_setup(ofg_prec* P)
    int big = INT32_MAX;
    bad.upload(&big, 1);
    const int invert = (P->type == OFG_SSOR) ? 0 : 1;
-   if (n) {
+   if (P->wfwd.on) wave_diagonal(P, invert, bad.p);
+   else if (n) {
       diag_setup<<<grid_for(n, 256), 256, 0, stream()>>>(n, A->dpos.p, A->val.p, P->pivot.p, invert,
                                                          bad.p);
       count_launch();
@@ -1218,9 +1219,10 @@ void prec_setup(ofg_prec* P)
       }
    }
    P->status.zero();
-   fill_sentinel(P->t.p, n);
    if (P->wfwd.on) {
+      if (P->wfwd.ext) fill_sentinel(P->t.p, n);
       if (ilu) {
+         ensure_sell(A);
          wave_factor(P);
          check_status(P);
       }
@@ -1228,6 +1230,7 @@ void prec_setup(ofg_prec* P)
       wave_values(P, P->wbwd);
       return;
    }
+   fill_sentinel(P->t.p, n);
    fill_slot_values(A, P->fwd);
    fill_slot_values(A, P->bwd);
    if (ilu) {
