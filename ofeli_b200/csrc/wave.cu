@@ -3,8 +3,9 @@
 // one warp instead of a scan per 32 rows.
 //
 // A line is a maximal run of rows that each depend on the row just before.
-// Up to 31 consecutive lines form a group, one lane a line (lane 0 carries
-// the line before the group).  Lane l starts its line `shift` steps after
+// Up to 32 consecutive lines form a group, one lane a line; where the group's
+// first line depends on the line before, lane 0 carries that one and 31 lines
+// follow.  Lane l starts its line `shift` steps after
 // lane l - 1, so that at every step the value a row needs from the previous
 // line was computed one (slot A) or two (slot B) steps earlier by the
 // neighbouring lane, and the value of the row before (slot L) one step
@@ -52,7 +53,6 @@ namespace {
 constexpr int kWaveF = 8;        // steps per chunk
 constexpr int kWaveTile = 32;    // steps per tile, the unit of the bulk copies
 constexpr int kTileChunks = kWaveTile / kWaveF;
-constexpr int kWaveLines = 31;   // lines of a group: lane 0 carries the line before it
 constexpr int kWavePitch = 34;   // row pitch of the [step][lane] tiles: 8 steps x 2 lanes hit 16 banks once
 constexpr int kWaveCPitch = 68;  // the same for the pairs of the right-hand side
 constexpr int kExt = kWaveExt;
@@ -381,7 +381,8 @@ struct WaveRun {
 template <int MODE, bool FAST>
 __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int next, bool same_tile,
                                            uint32_t next_bar, unsigned next_phase, bool next_ok,
-                                           int j0, int len, int lane, double* edge_out,
+                                           int j0, int len, int lane, bool carry,
+                                           double* edge_out,
                                            WaveRun<wave_slots(MODE)>& R)
 {
    double cn[kWaveF];
@@ -392,7 +393,7 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
       const bool act = (unsigned)(j0 + s) < (unsigned)len;
       double zn = wave_step<MODE>(R.op.a[s % kAhead], R.op.c[s], R.u1, R.u2, R.z, act);
       if (!FAST && !act) zn = 0.0;
-      if ((!FAST || MODE == W_FACTOR) && lane == 0) zn = R.op.c[s];
+      if ((!FAST || MODE == W_FACTOR) && carry) zn = R.op.c[s];
       R.z = zn;
       R.u2 = R.u1;
       // (first of the step's shared-memory operations: the next step waits for it)
@@ -424,7 +425,8 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
 // lo, hi: the steps in which the fast form may be used.
 template <int MODE>
 __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, unsigned tiles,
-                                             int nch, int lane, const LineInfo& li, double* edge_out,
+                                             int nch, int lane, bool carry, const LineInfo& li,
+                                             double* edge_out,
                                              int lo, int hi)
 {
    WaveRun<wave_slots(MODE)> R;
@@ -438,7 +440,7 @@ __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, 
       wave_steps<MODE, decltype(fast)::value>(
          sh, at.slot, nx.slot, nx.tile == at.tile, smem_u32(&sh.full[nx.tile]), nx.phase,
          ch + 1 < nch && t0 + kWaveF >= lo && t0 + 2 * kWaveF <= hi && !special, t0 - li.shift,
-         li.len, lane, edge_out ? edge_out + t0 : nullptr, R);
+         li.len, lane, carry, edge_out ? edge_out + t0 : nullptr, R);
    };
    int ch = 0;
 #pragma unroll 1
@@ -523,26 +525,27 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
       const int ein = g.g_edge[grp];
       const int plen = ein >= 0 ? g.line[l0] - g.line[l0 - 1] : 0;
       const int sm1 = g.g_sm1[grp];
+      const int first = ein >= 0 ? 1 : 0;  // lane of the group's first line
       const int ntile = (nch + kTileChunks - 1) / kTileChunks;
 
       if (w == 0) {
          // ------------------------------------------------------- compute
-         const LineInfo li = wave_line(g, l0 + lane - 1, l0, l1);
+         const LineInfo li = wave_line(g, l0 + lane - first, l0, l1);
          // the group's last line goes on to the next group, entry j at step j + shift
          const int eo = grp + 1 < g.ngroups ? g.g_edge[grp + 1] : -1;
-         double* edge_out = eo >= 0 && lane == l1 - l0 ? g.edge + eo - li.shift : nullptr;
+         double* edge_out = eo >= 0 && lane == l1 - l0 - 1 + first ? g.edge + eo - li.shift : nullptr;
          // fast steps: all, or those in which every line is active
          const int lo = g.clean ? 0 : __reduce_max_sync(0xffffffffu, li.shift);
          const int hi = g.clean ? INT_MAX
                                 : __reduce_min_sync(0xffffffffu, li.len ? li.shift + li.len : INT_MAX);
-         wave_compute<MODE>(sh, g.status, tiles, nch, lane, li, edge_out, lo, hi);
+         wave_compute<MODE>(sh, g.status, tiles, nch, lane, first && lane == 0, li, edge_out, lo, hi);
       }
       else if (w == 1) {
          // ---------------------------------------------------------- feed
          LineInfo li[8];
          if (!EXT) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) li[q] = wave_line(g, l0 + 4 * q + (lane >> 3) - 1, l0, l1);
+            for (int q = 0; q < 8; ++q) li[q] = wave_line(g, l0 + 4 * q + (lane >> 3) - first, l0, l1);
          }
          for (int tl = 0; tl < ntile; ++tl) {
             const ChunkAt<MODE> at(tiles, tl * kTileChunks);
@@ -566,7 +569,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
                      const int j = t - li[q].shift;
                      const bool valid = (unsigned)j < (unsigned)li[q].len;
                      const int rho = li[q].start + (valid ? j : 0);
-                     if (4 * q + (lane >> 3) > 0)
+                     if (4 * q + (lane >> 3) >= first)
                         copy8(smem_u32(&sh.c[at.slot + cc][c_pos(tt, 4 * q + (lane >> 3))]),
                               g.in + (FWD ? rho : n - 1 - rho), valid);
                   }
@@ -580,8 +583,8 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          // ---------------------------------------- the line before the group
          // lane 0's right-hand side at step t: entry t - sm1 of that line,
          // zero outside it
-         double* src = g.edge + (ein >= 0 ? ein : 0);
-         for (int tl = 0; tl < ntile; ++tl) {
+         double* src = g.edge + (first ? ein : 0);
+         for (int tl = 0; first && tl < ntile; ++tl) {
             const ChunkAt<MODE> at(tiles, tl * kTileChunks);
             if (tiles + tl >= Sh::NT &&
                 !wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u, &sh.stop, g.status))
@@ -614,7 +617,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          const int f = w == 3 ? 0 : w - 4, tt = lane & 7;
          LineInfo li[8];
 #pragma unroll
-         for (int q = 0; q < 8; ++q) li[q] = wave_line(g, l0 + 4 * q + (lane >> 3) - 1, l0, l1);
+         for (int q = 0; q < 8; ++q) li[q] = wave_line(g, l0 + 4 * q + (lane >> 3) - first, l0, l1);
          // per row: the pivot that scales the result (forward: see wave_fill),
          // or the row's entry of dot_with
          const double* aux = FWD ? (MODE == W_FACTOR || EXT ? nullptr : g.piv) : g.dot_with;
@@ -730,10 +733,10 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          // ------------------------------------ right-hand side with E slots
          // four lines a warp, eight steps of each
          const int tt = lane & 7, ln = 4 * (w - 3 - NST) + (lane >> 3);
-         const LineInfo li = wave_line(g, l0 + ln - 1, l0, l1);
+         const LineInfo li = wave_line(g, l0 + ln - first, l0, l1);
          int32_t off[kExt];
 #pragma unroll
-         for (int k = 0; k < kExt; ++k) off[k] = li.len ? g.eoff[(l0 + ln - 1) * kExt + k] : 0;
+         for (int k = 0; k < kExt; ++k) off[k] = li.len ? g.eoff[(l0 + ln - first) * kExt + k] : 0;
          struct {
             double a[kExt], at[kExt], b, pv;
          } r;
@@ -814,7 +817,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
                for (int k = 0; k < kExt; ++k)
                   if (!wave_empty(r.a[k])) c = fma(-r.a[k], v[k], c);
             }
-            if (ln > 0) st_shared(&sh.c[at.slot][c_pos(tt, ln)], c);
+            if (ln >= first) st_shared(&sh.c[at.slot][c_pos(tt, ln)], c);
             fetch(ch + 1);
          }
       }
@@ -936,7 +939,7 @@ struct FillArgs {
    const int32_t* stpos;    // FACTOR: transposed positions (CSR) in SELL order
    const double* val;       // FACTOR: the CSR values
    const int32_t* tile_g;   // group of every layout tile
-   const int32_t *g_line, *g_tile, *line, *shift, *dshift, *eoff;
+   const int32_t *g_line, *g_tile, *g_edge, *line, *shift, *dshift, *eoff;
    const double* piv;       // solve: inverse pivots, or (ssor) the diagonal
    bool ssor;
    double* coef;
@@ -975,13 +978,14 @@ __global__ void __launch_bounds__(256) wave_fill(FillArgs f)
    const int t = blockIdx.x, g = f.tile_g[t];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    const int l0 = f.g_line[g], l1 = f.g_line[g + 1];
+   const int first = f.g_edge[g] >= 0 ? 1 : 0;  // lane of the group's first line
    const int step = (t - f.g_tile[g]) * kWaveTile + lane;
    for (int ln = w; ln < 32; ln += 8) {
       double s[NS];
 #pragma unroll
       for (int k = 0; k < NS; ++k) s[k] = 0.0;
-      const int l = l0 + ln - 1;
-      if (ln > 0 && l < l1) {
+      const int l = l0 + ln - first;
+      if (l >= l0 && l < l1) {
          const int32_t beg = f.line[l], len = f.line[l + 1] - beg;
          const int32_t pbeg = l > 0 ? f.line[l - 1] : beg;
          const int32_t ds = f.dshift[l];
@@ -1125,6 +1129,7 @@ FillArgs fill_args(const ofg_matrix* A, const WavePlan& p)
    f.tile_g = p.tile_g.p;
    f.g_line = p.g_line.p;
    f.g_tile = p.g_tile.p;
+   f.g_edge = p.g_edge.p;
    f.line = p.line.p;
    f.shift = p.shift.p;
    f.dshift = p.dshift.p;
@@ -1215,7 +1220,7 @@ bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpo
       if (e[0]) p.ext = true;
    }
    int64_t edge = 0, steps = 0;
-   int g0 = 0;
+   int g0 = 0, room = 32;
    auto close = [&](int l1) {
       if (l1 == g0) return;
       int32_t m = 0;
@@ -1244,9 +1249,10 @@ bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpo
       // lanes that have ended read it), so that no value, finite or not, needs
       // masking outside the lines
       if (coupled && (dshift[l] != 1 || line[l + 1] - line[l] != line[l] - line[l - 1])) p.clean = false;
-      if (l == 0 || l == g0 + kWaveLines || !coupled || eline >= g0) {
+      if (l == 0 || l == g0 + room || !coupled || eline >= g0) {
          close(l);
          g0 = l;
+         room = coupled ? 31 : 32;
          g_line.push_back(l);
          g_tile.push_back((int32_t)tile_g.size());
          if (coupled) {

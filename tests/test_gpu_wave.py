@@ -1,5 +1,5 @@
 """The wavefront sweeps (csrc/wave.cu): D-ILU pivots and Prec applications
-against the oracle at the edges of their groups (31 lines), tiles (32 steps)
+against the oracle at the edges of their groups (32 and 31 lines), tiles (32 steps)
 and chunks (8 steps), on shapes that take the wavefront's masked form (lines
 of unequal length, two steps apart) and on shapes that must be left to the
 general sweeps, with right-hand sides that are not finite."""
@@ -44,8 +44,9 @@ def cube(M):
 
 SHAPES = {
     "one_group": lambda: square(32, 9),          # 31 lines of 8
-    "two_groups": lambda: square(33, 40),        # 31 + 1 lines
-    "tiles": lambda: square(95, 258),            # 94 lines of 257
+    "full_group": lambda: square(33, 40),        # 32 lines
+    "two_groups": lambda: square(34, 40),        # 32 + 1 lines
+    "tiles": lambda: square(95, 258),            # 32 + 31 + 31 lines of 257
     "ragged": lambda: square(64, 171),
     "neumann": lambda: square(40, 33, (0, 1, 1, 0)),
     "wide": lambda: square(4, 700),              # few lanes: the general sweeps
@@ -55,9 +56,10 @@ SHAPES = {
     "stair_long": lambda: staircase(64, 200, 150),
     "cube_10": lambda: cube(10),
     "cube_32": lambda: cube(32),                 # planes of 31 lines
-    "cube_37": lambda: cube(37),
+    "cube_37": lambda: cube(37),                 # planes of 32 + 4 lines
     # more groups than blocks: a block goes on from group to group
-    "cube_64": lambda: cube(64),                 # planes of 31 + 31 + 1 lines
+    "cube_70": lambda: cube(70),                 # planes of 32 + 31 + 6 lines
+    "cube_64": lambda: cube(64),                 # planes of 32 + 31 lines
     "tall": lambda: square(4710, 27),
 }
 
