@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(kRedBlock, 8) gm_mgs(int64_t n, double* w,
                                                     const double* __restrict__ pin, double* pout,
                                                     const GMState* S)
 {
+   pdl_wait();
+   pdl_release();
    if (S->stop) return;
    double h = 0.0;
    if (hprev) {
@@ -275,6 +277,8 @@ __global__ void __launch_bounds__(kRedBlock, 8) gm_mgs_last(int64_t n, double* w
                                                          const double* __restrict__ pin,
                                                          double* pout, const GMState* S)
 {
+   pdl_wait();
+   pdl_release();
    if (S->stop) return;
    double tot[1];
    partials_total<1>(pin, gridDim.x, tot);
@@ -296,6 +300,8 @@ __global__ void __launch_bounds__(kRedBlock, 8) gm_scale(int64_t n, const double
                                                       const double* __restrict__ pin,
                                                       const GMState* S)
 {
+   pdl_wait();
+   pdl_release();
    if (S->stop) return;
    double tot[1];
    partials_total<1>(pin, gridDim.x, tot);
@@ -338,6 +344,8 @@ __device__ __forceinline__ void set_rotation(double dx, double dy, double& cs, d
 __global__ void gm_givens(double* H, double* s, double* cs, double* sn, int i, int m, GMState* S,
                           double tol, int max_it)
 {
+   pdl_wait();
+   pdl_release();
    if (S->stop || threadIdx.x != 0) return;
    const int ld = m + 1;
    for (int k = 0; k < i; ++k) rotate(H[k * ld + i], H[(k + 1) * ld + i], cs[k], sn[k]);
@@ -532,19 +540,16 @@ void gmres_solve(ofg_prec* P, const double* b, double* x, int m, int max_it, dou
             precond_inplace(w.p, &S.p->stop);
             // gm_mgs(k) writes gpb[k & 1]; H(k-1,i) is stored by gm_mgs(k),
             // H(i,i) by gm_mgs_last, H(i+1,i) by gm_scale
-            for (int k = 0; k <= i; ++k) {
-               gm_mgs<<<g, kRedBlock, 0, stream()>>>(
-                  n, w.p, k > 0 ? V.p + (size_t)(k - 1) * n : nullptr,
-                  k > 0 ? H.p + (size_t)(k - 1) * ld + i : nullptr, V.p + (size_t)k * n,
-                  gpb[(k + 1) & 1], gpb[k & 1], S.p);
-            }
-            gm_mgs_last<<<g, kRedBlock, 0, stream()>>>(n, w.p, vi, H.p + (size_t)i * ld + i,
-                                                       gpb[i & 1], gpb[(i + 1) & 1], S.p);
-            gm_scale<<<g, kRedBlock, 0, stream()>>>(n, w.p, V.p + (size_t)(i + 1) * n,
-                                                    H.p + (size_t)(i + 1) * ld + i,
-                                                    gpb[(i + 1) & 1], S.p);
-            gm_givens<<<1, 32, 0, stream()>>>(H.p, s.p, cs.p, sn.p, i, m, S.p, tol, max_it);
-            count_launch(i + 5);
+            // (each kernel of the chain starts while the one before drains)
+            for (int k = 0; k <= i; ++k)
+               launch_pdl(gm_mgs, g, kRedBlock, n, w.p, k > 0 ? V.p + (size_t)(k - 1) * n : nullptr,
+                          k > 0 ? H.p + (size_t)(k - 1) * ld + i : nullptr, V.p + (size_t)k * n,
+                          gpb[(k + 1) & 1], gpb[k & 1], S.p);
+            launch_pdl(gm_mgs_last, g, kRedBlock, n, w.p, vi, H.p + (size_t)i * ld + i, gpb[i & 1],
+                       gpb[(i + 1) & 1], S.p);
+            launch_pdl(gm_scale, g, kRedBlock, n, w.p, V.p + (size_t)(i + 1) * n,
+                       H.p + (size_t)(i + 1) * ld + i, gpb[(i + 1) & 1], S.p);
+            launch_pdl(gm_givens, 1, 32, H.p, s.p, cs.p, sn.p, i, m, S.p, tol, max_it);
             OFG_LAUNCH_CHECK();
          }
          if (i < m) {
