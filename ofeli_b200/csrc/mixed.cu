@@ -481,6 +481,17 @@ struct SliceValues {
    ValueTab get() const { return ValueTab{head.p, tab.p}; }
 };
 
+// The tables pay once what an iteration streams no longer stays in the L2's
+// near half (the values then come from DRAM or the far half); below, the table
+// loads are a longer chain than the values' own.  Measured per solve, without
+// and with the table of A: 37 MB (800^2, learned) 65.2 / 65.2 ms, 34 MB
+// (1000^2, Jacobi) 98.1 / 98.5, 50 MB (1000 x 700, learned) 103.6 / 95.9,
+// 49 MB (1200^2, Jacobi) 163 / 136; without and with those of G and G^T, the
+// values of A no longer counted: 44 MB (1000^2) 86.7 / 87.0, 52 MB
+// (1100 x 1090) 108.6 / 110.5, 63 MB (1200^2) 124.0 / 120.6, 69 MB
+// (1300 x 1203) 245 / 228.
+constexpr double kTableSetA = 45e6, kTableSetG = 60e6;
+
 // Worth it from half of the entries on
 bool mostly_shared(const ofg_matrix* M, unsigned long long shared)
 {
@@ -573,17 +584,26 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
    SliceValues av, lv, uv;
    DBuf<unsigned long long> shared(3);
    shared.zero();
-   if (auni && inner_bits != 16) av.scan(A, A->sell_val.p, shared.p);
+   // bytes an iteration streams besides the values of A
+   const double set_g =
+      index_bytes(A, a16, auni) + 4.0 * n * (learned ? 7 : 5) +
+      (learned ? 2.0 * (LP->gl->nnz + LP->gu->nnz) + index_bytes(LP->gl, g16, luni) +
+                    index_bytes(LP->gu, g16, uuni)
+               : 0.0);
+   const bool try_a = auni && inner_bits != 16 && set_g + 4.0 * A->nnz >= kTableSetA;
+   const bool try_g = set_g >= kTableSetG;
+   if (try_a) av.scan(A, A->sell_val.p, shared.p);
    using bf16 = __nv_bfloat16;
-   if (luni) lv.scan(LP->gl, reinterpret_cast<const bf16*>(LP->gl->sell_valbf.p), shared.p + 1);
-   if (uuni) uv.scan(LP->gu, reinterpret_cast<const bf16*>(LP->gu->sell_valbf.p), shared.p + 2);
+   if (luni && try_g) lv.scan(LP->gl, reinterpret_cast<const bf16*>(LP->gl->sell_valbf.p), shared.p + 1);
+   if (uuni && try_g) uv.scan(LP->gu, reinterpret_cast<const bf16*>(LP->gu->sell_valbf.p), shared.p + 2);
    int hb[2] = {0, 0};
    unsigned long long hs[3] = {0, 0, 0};
    OFG_CUDA(cudaMemcpyAsync(hs, shared.p, sizeof(hs), cudaMemcpyDeviceToHost, stream()));
    bad.download(hb, 2);
-   const bool aval = auni && inner_bits != 16 && mostly_shared(A, hs[0]);
-   const bool lval = luni && mostly_shared(LP->gl, hs[1]);
-   const bool uval = uuni && mostly_shared(LP->gu, hs[2]);
+   const double a_bytes = inner_bits == 0 && !hb[1] ? 2.0 : 4.0;  // per value of A
+   const bool aval = try_a && set_g + a_bytes * A->nnz >= kTableSetA && mostly_shared(A, hs[0]);
+   const bool lval = luni && try_g && mostly_shared(LP->gl, hs[1]);
+   const bool uval = uuni && try_g && mostly_shared(LP->gu, hs[2]);
    OFG_REQUIRE(!hb[0], OFG_ERR_PIVOT, "zero diagonal entry");
    int bits = inner_bits;
    if (inner_bits == 0) {
