@@ -185,33 +185,33 @@ __global__ void __launch_bounds__(kRedBlock, kQuadBlocks) mx_spmv(int64_t nquads
          acc = value_quad(vt.tab + hd.x, hd.y, p, (int)r0);
       }
       else {
-      const int32_t beg = sp[s], w = (sp[s + 1] - beg) >> 5;
-      const T* vp = sval + beg + lane0;
-      const int32_t u = UNI ? suni[s] : -1;
-      if (u >= 0) {
-         acc = uniform_quad(vp, stab + u, w, p, (int)r0);
-      }
-      else {
-         const I* cp = scol + beg + lane0;
-         auto step = [&](int32_t k) {
-            const int4 c = load_cols(cp + k * 32, r0);
-            const float4 a = load_vals(vp + k * 32);
-            acc.x += a.x * __ldg(p + c.x);
-            acc.y += a.y * __ldg(p + c.y);
-            acc.z += a.z * __ldg(p + c.z);
-            acc.w += a.w * __ldg(p + c.w);
-         };
-         // with uniform slices this path is the rare one: kept rolled so
-         // that it does not set the kernel's register count
-         if (UNI) {
-#pragma unroll 1
-            for (int32_t k = 0; k < w; ++k) step(k);
+         const int32_t beg = sp[s], w = (sp[s + 1] - beg) >> 5;
+         const T* vp = sval + beg + lane0;
+         const int32_t u = UNI ? suni[s] : -1;
+         if (u >= 0) {
+            acc = uniform_quad(vp, stab + u, w, p, (int)r0);
          }
          else {
+            const I* cp = scol + beg + lane0;
+            auto step = [&](int32_t k) {
+               const int4 c = load_cols(cp + k * 32, r0);
+               const float4 a = load_vals(vp + k * 32);
+               acc.x += a.x * __ldg(p + c.x);
+               acc.y += a.y * __ldg(p + c.y);
+               acc.z += a.z * __ldg(p + c.z);
+               acc.w += a.w * __ldg(p + c.w);
+            };
+            // with uniform slices this path is the rare one: kept rolled so
+            // that it does not set the kernel's register count
+            if (UNI) {
+#pragma unroll 1
+               for (int32_t k = 0; k < w; ++k) step(k);
+            }
+            else {
 #pragma unroll 8
-            for (int32_t k = 0; k < w; ++k) step(k);
+               for (int32_t k = 0; k < w; ++k) step(k);
+            }
          }
-      }
       }
       *reinterpret_cast<float4*>(q + r0) = acc;
       const float4 pr = *reinterpret_cast<const float4*>(p + r0);

@@ -3,7 +3,13 @@
 // SpMatrix::DILUSolve / SSORSolve (include/linear_algebra/SpMatrix_impl.h
 // :882-942) and the pivot recurrence of DILUFactorize (:837-870).
 //
-// Sweep scheduling.  Rows keep OFELI's natural order, so the preconditioner
+// Two forms of the sweeps.  Matrices whose rows form long grid lines with at
+// most three couplings to the line itself and the one before (structured
+// meshes in natural order) take the wavefront of wave.cu, both directions or
+// none; every other matrix (unstructured files, short or ragged lines) takes
+// the sweeps of this file.
+//
+// Sweep scheduling here.  Rows keep OFELI's natural order, so the preconditioner
 // is the reference's own.  Rows are cut into strands: maximal runs of
 // consecutive rows where each row depends on the row just before it (on a
 // structured mesh one strand is one grid line of unknowns).  A warp takes
@@ -1152,6 +1158,7 @@ void check_status(ofg_prec* P)
       P->status.zero();
       wave_repair(P->wfwd);
       wave_repair(P->wbwd);
+      if (P->t.p) fill_sentinel(P->t.p, (int64_t)P->t.n);
       throw Error(OFG_ERR_TIMEOUT, "triangular sweep wait ran out (status " + std::to_string(h) + ")");
    }
 }

@@ -78,10 +78,7 @@ constexpr int kHoist = 1;
 // register budget: 65536 / (256 * kQuadBlocks)), and the grid of the
 // kernel chains they are part of.
 constexpr int kQuadBlocks = 8;
-#ifndef KVU
-#define KVU 1
-#endif
-constexpr int kValueUnroll = KVU;
+constexpr int kValueUnroll = 1;
 
 // The four rows r0 .. r0+3 of a uniform slice: w positions, the offset of
 // position k from tp[k].  The values of kHoist positions are loaded before

@@ -15,14 +15,16 @@
 // right-hand side by loader warps.
 //
 // What bounds it: the dependency chain, (columns + lines) steps and one
-// hand-off per group.  A step takes 66 to 70 cycles (shuffle 24 and a
-// dependent FP64 operation 8, measured; the rest is the shared-memory traffic
-// around it), a hand-off between SMs about 3000 (one-way latency 530 to 1070,
-// measured, plus the chunk it travels in).  At 2049^2 a solve sweep takes
-// 250 us where the sweeps of prec.cu, which resolve 32 rows of a line by a
-// scan, took 1040; the factorisation 0.54 instead of 13.4 ms.  On the 129^3
-// cube a sweep takes 330 instead of 530 us: there the chain is 127 planes of
-// about 2.6 us, a chunk of steps and a trip through L2 each.
+// hand-off per group.  A step's chain is a shuffle (24 cycles, measured) and
+// three dependent FP64 operations (8 each); with the shared-memory traffic
+// around it a step takes about 90 cycles (the sweep's time less the
+// hand-offs).  A hand-off between SMs takes about 3000 (one-way latency 530
+// to 1070, measured, plus the chunk it travels in).  At 2049^2 a solve sweep
+// takes 294 us where the sweeps of prec.cu, which resolve 32 rows of a line
+// by a scan, took 1040; the factorisation 0.56 instead of 13.4 ms.  On the
+// 129^3 cube a sweep takes 365 instead of 530 us, the factorisation 0.44
+// instead of 4.6 ms: there the chain is 127 planes of about 2.6 us, a chunk
+// of steps and a trip through L2 each.
 //
 // One block works on a group at a time, its warps in roles:
 //   * warp 0 computes, kWaveF steps (a chunk) at a time, from shared memory;
@@ -597,7 +599,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
             if (there && !todo) st_shared(dst, 0.0);
             const unsigned long long w0 = global_ns();
             for (unsigned spins = 1; __any_sync(0xffffffffu, todo); ++spins) {
-               if (todo) {  // (32 bytes x 8 per poll: no back-off needed)
+               if (todo) {
                   const double v = ld_relaxed(src + i);
                   if (!wave_empty(v)) {
                      st_shared(dst, v);
