@@ -582,8 +582,7 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
    count_launch();
    // slices that share their values, in A (not in the lossy BF16 copy), G, G^T
    SliceValues av, lv, uv;
-   DBuf<unsigned long long> shared(3);
-   shared.zero();
+   DBuf<unsigned long long> shared;
    // bytes an iteration streams besides the values of A
    const double set_g =
       index_bytes(A, a16, auni) + 4.0 * n * (learned ? 7 : 5) +
@@ -592,13 +591,19 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
                : 0.0);
    const bool try_a = auni && inner_bits != 16 && set_g + 4.0 * A->nnz >= kTableSetA;
    const bool try_g = set_g >= kTableSetG;
+   const bool scan = try_a || (try_g && (luni || uuni));
+   if (scan) {
+      shared.alloc(3);
+      shared.zero();
+   }
    if (try_a) av.scan(A, A->sell_val.p, shared.p);
    using bf16 = __nv_bfloat16;
    if (luni && try_g) lv.scan(LP->gl, reinterpret_cast<const bf16*>(LP->gl->sell_valbf.p), shared.p + 1);
    if (uuni && try_g) uv.scan(LP->gu, reinterpret_cast<const bf16*>(LP->gu->sell_valbf.p), shared.p + 2);
    int hb[2] = {0, 0};
    unsigned long long hs[3] = {0, 0, 0};
-   OFG_CUDA(cudaMemcpyAsync(hs, shared.p, sizeof(hs), cudaMemcpyDeviceToHost, stream()));
+   if (scan)
+      OFG_CUDA(cudaMemcpyAsync(hs, shared.p, sizeof(hs), cudaMemcpyDeviceToHost, stream()));
    bad.download(hb, 2);
    const double a_bytes = inner_bits == 0 && !hb[1] ? 2.0 : 4.0;  // per value of A
    const bool aval = try_a && set_g + a_bytes * A->nnz >= kTableSetA && mostly_shared(A, hs[0]);
