@@ -156,8 +156,10 @@ void assemble(ofg_mesh* m, ofg_matrix* A, const Elem& el, double* db, int node_f
    OFG_CUDA(cudaMemsetAsync(bad.p, 0xFF, sizeof(unsigned), stream()));
    if (m->nn) {
       const int nen = m->nen;
-      double bytes = 4.0 * (m->nn + 1) + 8.0 * nen * m->ne + 8.0 * m->dim * m->nn + 8.0 * m->nn +
-                     4.0 * nen * nen * m->ne + 8.0 * node_fields * m->nn +
+      // records, or node-to-element lists, connectivity and element-to-CSR map
+      const double lists = A->inc_on ? (nen == 3 ? 16.0 : 20.0) * nen * m->ne
+                                     : 4.0 * (m->nn + 1) + 8.0 * nen * m->ne + 4.0 * nen * nen * m->ne;
+      double bytes = lists + 8.0 * m->dim * m->nn + 8.0 * m->nn + 8.0 * node_fields * m->nn +
                      8.0 * elem_fields * m->ne + 4.0 * (A->n + 1) +
                      8.0 * A->nnz + 8.0 * A->n;
       int* worked = prof_begin();
