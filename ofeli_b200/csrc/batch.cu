@@ -139,11 +139,9 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, unsigned rank)
    return r;
 }
 
-__device__ __forceinline__ double ld_cluster(const double* p, unsigned rank)
+__device__ __forceinline__ void st_cluster(double* p, unsigned rank, double v)
 {
-   double v;
-   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
-   return v;
+   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(p, rank)), "d"(v) : "memory");
 }
 
 __device__ __forceinline__ int ld_cluster(const int* p, unsigned rank)
@@ -156,13 +154,19 @@ __device__ __forceinline__ int ld_cluster(const int* p, unsigned rank)
 // The blocks working on one problem: one block (size 1: block barriers and
 // block reductions), or the whole cluster (size > 1: each block owns a
 // contiguous share of rows, nonzeros and nodes; cluster
-// barriers; reductions summed over the blocks in rank order through
-// distributed shared memory, double-buffered exchange slots).
+// barriers; reductions summed over the blocks in rank order).  In a cluster
+// each block's first warp stores its totals into every block's slots, and the
+// cluster barrier that follows is the block's own as well: 8 problems of up to
+// 4000 nodes in clusters of 8 take 2.65 ms, 24 of up to 32000 14.1; with all
+// threads reading the other blocks' slots after the barrier 3.31 and 15.8.
+// The slots are double-buffered: those of a sum are stored into again two
+// barriers after its own.
+constexpr int kMaxCluster = 8;
 template <int THREADS>
 struct Team {
    int rank, size;
    double (*sh)[THREADS / 32];
-   double (*xr)[4];
+   double (*xr)[kMaxCluster][3];
    int parity;
    __device__ __forceinline__ void bar()
    {
@@ -172,20 +176,32 @@ struct Team {
    template <int NV>
    __device__ __forceinline__ void sum(double (&v)[NV])
    {
-      block_sum<NV, THREADS>(v, sh);
-      if (size > 1) {
-         if (threadIdx.x == 0)
+      if (size == 1) {
+         block_sum<NV, THREADS>(v, sh);
+         return;
+      }
+      const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-            for (int i = 0; i < NV; ++i) xr[parity][i] = v[i];
-         cluster_sync();
+      for (int i = 0; i < NV; ++i) {
+         const double s = warp_sum(v[i]);
+         if (lane == 0) sh[i][w] = s;
+      }
+      __syncthreads();
+      if (w == 0) {
 #pragma unroll
          for (int i = 0; i < NV; ++i) {
-            double s = 0.0;
-            for (int r = 0; r < size; ++r) s += ld_cluster(&xr[parity][i], (unsigned)r);
-            v[i] = s;
+            const double s = warp_sum(lane < THREADS / 32 ? sh[i][lane] : 0.0);
+            if (lane < size) st_cluster(&xr[parity][rank][i], (unsigned)lane, s);
          }
-         parity ^= 1;
       }
+      cluster_sync();
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+         double s = 0.0;
+         for (int r = 0; r < size; ++r) s += xr[parity][r][i];
+         v[i] = s;
+      }
+      parity ^= 1;
    }
    __device__ __forceinline__ int64_t lo(int64_t n) const { return n * rank / size; }
    __device__ __forceinline__ int64_t hi(int64_t n) const { return n * (rank + 1) / size; }
@@ -609,7 +625,7 @@ __global__ void __launch_bounds__(THREADS, kResident / THREADS) batch_kernel(Bat
 {
    __shared__ int s_item;
    __shared__ double sh[3][THREADS / 32];
-   __shared__ double xr[2][4];
+   __shared__ double xr[2][kMaxCluster][3];
    const int tid = threadIdx.x;
    const unsigned rank = CS > 1 ? cluster_rank() : 0u;
    Team<THREADS> T{0, 1, sh, xr, 0};
@@ -927,15 +943,15 @@ void plan_items(ofg_batch* B, int config, std::vector<int32_t>& order,
 // alone or in clusters of 4 or 8, whichever ends first by a model of one
 // iteration, rows per thread plus a constant for its barriers (fitted to 8
 // and 24 problems of up to 4000 and 32000 nodes: 2.7 row steps in one block,
-// 3.7 and 4.6 in clusters), times rows^(1/2) iterations, over the items in
+// 3.3 and 3.55 in clusters), times rows^(1/2) iterations, over the items in
 // their order.  One block per problem leaves the launch waiting for the
 // largest one; with clusters, measured: 24 problems of 1000 to 32000 nodes
-// 60.0 (alone), 21.8 (4), 15.7 ms (8); 192 of them 100.2, 52.1, 58.5; but
-// 192 of 1000 to 4500 5.5, 8.2, 13.8.
+// 60.0 (alone), 21.2 (4), 14.1 ms (8); 192 of them 100.2, 50.2, 53.0; but
+// 192 of 1000 to 4500 5.5, 7.5, 11.8.
 int choose_config(ofg_batch* B)
 {
    constexpr int candidate[] = {4, 10, 16};
-   constexpr double barriers[] = {2.7, 3.7, 4.6};
+   constexpr double barriers[] = {2.7, 3.3, 3.55};
    int best = candidate[0];
    double least = 0.0;
    for (int c = 0; c < 3; ++c) {
