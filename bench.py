@@ -525,7 +525,9 @@ def measure(args, wl, R, work_stream, dev, world, rank, with_cpu=True):
     uniform = cnt and tot_bytes / cnt < ((4.0 if bits == 32 else 2.0) + 2.0) * A.nnz + 12.0 * n
     traffic = ncu_traffic(("mx_spmv_f32" if bits == 32 else "mx_spmv_bf16") +
                           ("_uniform" if uniform else ""))
-    if wl != "poisson2d":
+    # slices with a value table stream no values: no capture of that form
+    tables = cnt and tot_bytes / cnt < (4.0 if bits == 32 else 2.0) * A.nnz + 12.0 * n
+    if wl != "poisson2d" or tables:
         traffic = None  # the committed capture is of the 2-D matrix
     cpu = None
     if world == 1 and wl == "poisson2d":

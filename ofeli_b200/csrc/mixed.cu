@@ -639,8 +639,15 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
    // algorithmic bytes of the two factor products: BF16 value + column
    // index (2 or 4 bytes) per entry, the gathered input and the output (and
    // r, q for the reduction of the second)
-   const double gl_bytes = learned ? 2.0 * LP->gl->nnz + index_bytes(LP->gl, g16, luni) : 0.0;
-   const double gu_bytes = learned ? 2.0 * LP->gu->nnz + index_bytes(LP->gu, g16, uuni) : 0.0;
+   // a slice with a value table streams none of its values
+   auto streamed = [](const ofg_matrix* M, double each, bool table, unsigned long long in_table) {
+      if (!table) return each * (double)M->nnz;
+      return each * (double)std::max<int64_t>(0, M->nnz - (int64_t)in_table) + 8.0 * M->nslices;
+   };
+   const double gl_bytes =
+      learned ? streamed(LP->gl, 2.0, lval, hs[1]) + index_bytes(LP->gl, g16, luni) : 0.0;
+   const double gu_bytes =
+      learned ? streamed(LP->gu, 2.0, uval, hs[2]) + index_bytes(LP->gu, g16, uuni) : 0.0;
    auto learned_direction = [&](int fresh, int upd_d, int it, int decide, const StopRule& st) {
       using bf = __nv_bfloat16;
       const bf* vl = reinterpret_cast<const bf*>(learned ? LP->gl->sell_valbf.p : nullptr);
@@ -765,8 +772,8 @@ void solve_mixed(ofg_matrix* A, int prec_type, int inner_bits, int mode, const d
             // as a 16-bit offset, or a uniform slice's table) per entry, p
             // gathered, q written, p read for the dot
             prof_end(bits == 32 ? PROF_SPMV32 : PROF_SPMV16,
-                     (bits == 32 ? 4.0 : 2.0) * A->nnz + index_bytes(A, a16, auni) + 12.0 * n +
-                        4.0);
+                     streamed(A, bits == 32 ? 4.0 : 2.0, aval, hs[0]) + index_bytes(A, a16, auni) +
+                        12.0 * n + 4.0);
             if (learned) {
                launch_pdl(mx_update<false>, gq, kRedBlock, nquads, rr.p, q.p, jac, S.p, pq,
                           rpart, cur);
