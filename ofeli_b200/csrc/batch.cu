@@ -20,8 +20,8 @@
 // through distributed shared memory -- and smaller problems are taken one
 // per block of the cluster, so that the largest problems no longer set the
 // length of the launch.  The launch shape -- threads per block, lanes per
-// row in the SpMV, blocks per cluster -- is picked from the problems' sizes,
-// or by a measured autotuner (ofg_batch_tune) that first measures every problem's work (rows
+// CSR row in the SpMV, blocks per cluster -- is picked from the problems'
+// sizes, or by a measured autotuner (ofg_batch_tune) that first measures every problem's work (rows
 // x iterations).  The launch (with the queue reset) is captured in a CUDA
 // graph and replayed.
 #include <algorithm>
@@ -39,7 +39,7 @@ namespace {
 using namespace elem;
 
 struct BatchProblem {
-   int64_t node_off, elem_off, row_off, rp_off, nnz_off, n2p_off, n2e_off, slice_off;
+   int64_t node_off, elem_off, row_off, rp_off, nnz_off, n2p_off, n2e_off;
    int32_t nn, ne, n, pad;
 };
 
@@ -65,15 +65,9 @@ struct BatchArgs {
    const int32_t* emap;
    // matrices and vectors
    const int32_t* row_ptr;
+   const int32_t* col;
    const int32_t* dpos;
    double* val;
-   // the same matrices in slices of 32 rows (see Slices): first position of
-   // each slice, per problem one more than its slices; columns as 16-bit
-   // offsets from the row, or absolute where an offset does not fit
-   const int32_t* slice_ptr;
-   const int16_t* soff;
-   const int32_t* scol;
-   double* sval;
    double *b, *x, *r, *p, *q, *dinv;
    // inputs and outputs
    const double* kel;
@@ -85,9 +79,11 @@ struct BatchArgs {
    int* bad;
    int max_it;
    double tol;
-   // mixed precision: FP32 values in slices, FP32 inner vectors
-   int mixed;
-   float* sval32;
+   // mixed precision: FP32 values, 16-bit column offsets (or int32 columns
+   // where an offset does not fit), FP32 inner vectors
+   int mixed, offsets16;
+   float* val32;
+   const int16_t* d16;
    float *rl, *pl, *ql, *dl, *dinv32;
 };
 
@@ -156,9 +152,9 @@ __device__ __forceinline__ int ld_cluster(const int* p, unsigned rank)
 // contiguous share of rows, nonzeros and nodes; cluster
 // barriers; reductions summed over the blocks in rank order).  In a cluster
 // each block's first warp stores its totals into every block's slots, and the
-// cluster barrier that follows is the block's own as well: 8 problems of up to
-// 4000 nodes in clusters of 8 take 2.65 ms, 24 of up to 32000 14.1; with all
-// threads reading the other blocks' slots after the barrier 3.31 and 15.8.
+// cluster barrier that follows is the block's own as well: with all threads
+// reading the other blocks' slots after the barrier, 8 problems of up to 4000
+// nodes took 25 % longer, 24 of up to 32000 12 % (1024 threads, clusters of 8).
 // The slots are double-buffered: those of a sum are stored into again two
 // barriers after its own.
 constexpr int kMaxCluster = 8;
@@ -205,114 +201,61 @@ struct Team {
    }
    __device__ __forceinline__ int64_t lo(int64_t n) const { return n * rank / size; }
    __device__ __forceinline__ int64_t hi(int64_t n) const { return n * (rank + 1) / size; }
-   // rows: whole slices of 32
-   __device__ __forceinline__ int row_lo(int n, int r) const
-   {
-      const int64_t ns = (n + 31) >> 5;
-      return (int)min((int64_t)n, 32 * (ns * r / size));
-   }
 };
 
-// A problem's matrix in slices of 32 consecutive rows, position k of a slice
-// holding the k-th entry of each of its rows side by side: neighbouring lanes
-// read neighbouring entries.  ptr counts positions.  Short rows are padded
-// (and the padding is not read).
-template <class V>
-struct Slices {
-   const int32_t* ptr;
-   const int16_t* off;   // columns as offsets from the row, or null
-   const int32_t* col;
-   const V* val;
-   __device__ __forceinline__ Slices(const BatchArgs& a, const BatchProblem& P, const V* values)
-       : ptr(a.slice_ptr + P.slice_off), off(a.soff), col(a.scol), val(values)
-   {
-   }
-};
-
-// (A x)_i of a row in slice positions [c0, c1), this lane's share of the LPR
-// lanes of the row, k ascending.  kAhead entries' loads go out together.
-constexpr int kAhead = 4;
-template <int LPR, class V>
-__device__ __forceinline__ V row_product(const Slices<V>& S, const V* x, int i, int c0, int c1,
-                                         int lane)
-{
-   V s = 0;
-   for (int k = c0 + lane; k < c1; k += kAhead * LPR) {
-      const int64_t at = 32 * (int64_t)k + (i & 31);
-      int c[kAhead];
-      V v[kAhead], xv[kAhead];
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) {
-         const bool in = k + j * LPR < c1;
-         c[j] = i;
-         v[j] = 0;
-         if (in) {
-            c[j] = S.off ? i + S.off[at + 32 * LPR * j] : S.col[at + 32 * LPR * j];
-            v[j] = S.val[at + 32 * LPR * j];
-         }
-      }
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) xv[j] = x[c[j]];
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j)
-         if (k + j * LPR < c1) s += v[j] * xv[j];
-   }
-   return s;
-}
-
-// row(i, (A x)_i) for the rows [r0, r1), LPR lanes per row (called by the
-// first of them)
-template <int THREADS, int LPR, class V, class Row>
-__device__ __forceinline__ void block_rows(int r0, int r1, const Slices<V>& S, const V* x, Row row)
+// y = A x over rows [r0, r1), LPR lanes per row; adds this thread's share of
+// (w, y) to wy (w may be null) and, when b != null, of ||b - y||^2 to rr
+// with b - y stored into rout
+template <int THREADS, int LPR>
+__device__ __forceinline__ void block_spmv(int r0, int r1, const int32_t* rp, const int32_t* col,
+                                           const double* val, const double* x, double* y,
+                                           const double* w, double& wy, const double* b,
+                                           double* rout, double& rr)
 {
    const int lane = threadIdx.x % LPR;
-   int i = r0 + (int)threadIdx.x / LPR;
-   int c0 = 0, c1 = 0;
-   if (i < r1) {
-      c0 = S.ptr[i >> 5];
-      c1 = S.ptr[(i >> 5) + 1];
-   }
-   for (int i0 = r0; i0 < r1; i0 += THREADS / LPR, i += THREADS / LPR) {
-      const int n = i + THREADS / LPR;
-      int n0 = 0, n1 = 0;
-      if (n < r1) {
-         n0 = S.ptr[n >> 5];
-         n1 = S.ptr[(n >> 5) + 1];
-      }
-      V s = i < r1 ? row_product<LPR>(S, x, i, c0, c1, lane) : (V)0;
+   for (int i0 = r0; i0 < r1; i0 += THREADS / LPR) {
+      const int i = i0 + (int)threadIdx.x / LPR;
+      double s = 0.0;
+      if (i < r1)
+         for (int k = rp[i] + lane; k < rp[i + 1]; k += LPR) s += val[k] * x[col[k]];
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
-      if (i < r1 && lane == 0) row(i, s);
-      c0 = n0;
-      c1 = n1;
+      if (i < r1 && lane == 0) {
+         if (y) y[i] = s;
+         if (w) wy += w[i] * s;
+         if (b) {
+            const double t = b[i] - s;
+            rout[i] = t;
+            rr += t * t;
+         }
+      }
    }
 }
 
-// r = b - A x over rows [r0, r1); this thread's share of ||r||^2
+// q = A p over rows [r0, r1) with FP32 values and FP32 vectors, columns as
+// 16-bit offsets from the row (d16) or absolute (col); adds this thread's
+// share of (p, q) to pq
 template <int THREADS, int LPR>
-__device__ __forceinline__ double block_residual(int r0, int r1, const Slices<double>& S,
-                                                 const double* x, const double* b, double* r)
+__device__ __forceinline__ void block_spmv32(int r0, int r1, const int32_t* rp, const int16_t* d16,
+                                             const int32_t* col, const float* val, const float* x,
+                                             float* y, double& pq)
 {
-   double rr = 0.0;
-   block_rows<THREADS, LPR>(r0, r1, S, x, [&](int i, double s) {
-      const double t = b[i] - s;
-      r[i] = t;
-      rr += t * t;
-   });
-   return rr;
-}
-
-// load(i, j), then store(i, j) for this thread's rows of [r0, r1), the loads of
-// two rows (j = 0, 1) before the stores of the first: one load latency per pair
-template <int THREADS, class Load, class Store>
-__device__ __forceinline__ void for_rows(int r0, int r1, Load load, Store store)
-{
-   for (int i = r0 + (int)threadIdx.x; i < r1; i += 2 * THREADS) {
-      const bool two = i + THREADS < r1;
-      load(i, 0);
-      if (two) load(i + THREADS, 1);
-      store(i, 0);
-      if (two) store(i + THREADS, 1);
+   const int lane = threadIdx.x % LPR;
+   for (int i0 = r0; i0 < r1; i0 += THREADS / LPR) {
+      const int i = i0 + (int)threadIdx.x / LPR;
+      float s = 0.f;
+      if (i < r1) {
+         if (d16)
+            for (int k = rp[i] + lane; k < rp[i + 1]; k += LPR) s += val[k] * x[i + d16[k]];
+         else
+            for (int k = rp[i] + lane; k < rp[i + 1]; k += LPR) s += val[k] * x[col[k]];
+      }
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
+      if (i < r1 && lane == 0) {
+         y[i] = s;
+         pq += (double)x[i] * (double)s;
+      }
    }
 }
 
@@ -327,9 +270,11 @@ __device__ void cg_mixed(const BatchArgs& a, const BatchProblem& P, Team<THREADS
                          int r1, int& it_out, double& res_out, bool& done_out)
 {
    const int tid = threadIdx.x;
+   const int32_t* rp = a.row_ptr + P.rp_off;
+   const int32_t* col = a.col + P.nnz_off;
    const double* val = a.val + P.nnz_off;
-   const Slices<double> A(a, P, a.sval);
-   const Slices<float> A32(a, P, a.sval32);
+   const float* v32 = a.val32 + P.nnz_off;
+   const int16_t* d16 = a.offsets16 ? a.d16 + P.nnz_off : nullptr;
    const double* b = a.b + P.row_off;
    double* x = a.x + P.row_off;
    double* r = a.r + P.row_off;
@@ -363,30 +308,17 @@ __device__ void cg_mixed(const BatchArgs& a, const BatchProblem& P, Team<THREADS
    while (!done && it < a.max_it) {
       ++it;
       double w1[1] = {0.0};
-      block_rows<THREADS, LPR>(r0, r1, A32, pl, [&](int i, float s) {
-         ql[i] = s;
-         w1[0] += (double)pl[i] * (double)s;
-      });
+      block_spmv32<THREADS, LPR>(r0, r1, rp, d16, col, v32, pl, ql, w1[0]);
       T.sum(w1);
       const float alpha = (float)(rho / w1[0]);
       double u2[2] = {0.0, 0.0};
-      float v0[2], v1[2], v2[2], v3[2], v4[2];
-      for_rows<THREADS>(
-         r0, r1,
-         [&](int i, int j) {
-            v0[j] = rl[i];
-            v1[j] = ql[i];
-            v2[j] = m32[i];
-            v3[j] = dl[i];
-            v4[j] = pl[i];
-         },
-         [&](int i, int j) {
-            dl[i] = v3[j] + alpha * v4[j];
-            const float ri = v0[j] - alpha * v1[j];
-            rl[i] = ri;
-            u2[0] += (double)ri * ri;
-            u2[1] += (double)ri * (ri * v2[j]);
-         });
+      for (int i = r0 + tid; i < r1; i += THREADS) {
+         dl[i] += alpha * pl[i];
+         const float ri = rl[i] - alpha * ql[i];
+         rl[i] = ri;
+         u2[0] += (double)ri * ri;
+         u2[1] += (double)ri * (ri * m32[i]);
+      }
       T.sum(u2);
       const double rn = sqrt(u2[0]);
       double rz = u2[1];
@@ -397,7 +329,8 @@ __device__ void cg_mixed(const BatchArgs& a, const BatchProblem& P, Team<THREADS
             dl[i] = 0.f;
          }
          T.bar();
-         double w2[1] = {block_residual<THREADS, LPR>(r0, r1, A, x, b, r)};
+         double w2[1] = {0.0}, d2 = 0.0;
+         block_spmv<THREADS, LPR>(r0, r1, rp, col, val, x, nullptr, nullptr, d2, b, r, w2[0]);
          T.sum(w2);
          res = sqrt(w2[0]) / bnorm;
          if (res <= a.tol) {
@@ -417,14 +350,7 @@ __device__ void cg_mixed(const BatchArgs& a, const BatchProblem& P, Team<THREADS
       }
       const float beta = (float)(rz / rho);
       rho = rz;
-      for_rows<THREADS>(
-         r0, r1,
-         [&](int i, int j) {
-            v0[j] = m32[i];
-            v1[j] = rl[i];
-            v2[j] = pl[i];
-         },
-         [&](int i, int j) { pl[i] = v0[j] * v1[j] + beta * v2[j]; });
+      for (int i = r0 + tid; i < r1; i += THREADS) pl[i] = m32[i] * rl[i] + beta * pl[i];
       T.bar();
    }
    if (!done && it > 0) {
@@ -434,7 +360,8 @@ __device__ void cg_mixed(const BatchArgs& a, const BatchProblem& P, Team<THREADS
          dl[i] = 0.f;
       }
       T.bar();
-      double w2[1] = {block_residual<THREADS, LPR>(r0, r1, A, x, b, r)};
+      double w2[1] = {0.0}, d2 = 0.0;
+      block_spmv<THREADS, LPR>(r0, r1, rp, col, val, x, nullptr, nullptr, d2, b, r, w2[0]);
       T.sum(w2);
       res = sqrt(w2[0]) / bnorm;
    }
@@ -454,6 +381,7 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
    const int32_t* code = a.code + P.node_off;
    const int32_t* dof = a.dof + P.node_off;
    const int32_t* rp = a.row_ptr + P.rp_off;
+   const int32_t* col = a.col + P.nnz_off;
    double* val = a.val + P.nnz_off;
    double* b = a.b + P.row_off;
    double* x = a.x + P.row_off;
@@ -461,8 +389,8 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
    double* p = a.p + P.row_off;
    double* q = a.q + P.row_off;
    double* dinv = a.dinv + P.row_off;
-   const Slices<double> A(a, P, a.sval);
-   const int r0 = T.row_lo(n, T.rank), r1 = T.row_lo(n, T.rank + 1);
+   const int nnz = rp[n];
+   const int r0 = (int)T.lo(n), r1 = (int)T.hi(n);
 
    // ---- Equation::build(): each node gathers its CSR row and RHS entry
    // over its elements in ascending order (the single-problem kernel's
@@ -490,21 +418,12 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
       T.bar();
    }
 
-   // ---- the values in slices (read after the sums that start the CG)
-   for (int i = r0 + tid; i < r1; i += THREADS) {
-      const int64_t at = 32 * (int64_t)A.ptr[i >> 5] + (i & 31);
-      const int k0 = rp[i], w = rp[i + 1] - k0;
-      for (int k = 0; k < w; ++k) {
-         const double v = val[k0 + k];
-         a.sval[at + 32 * (int64_t)k] = v;
-         if (a.mixed) a.sval32[at + 32 * (int64_t)k] = (float)v;
-      }
-   }
-
    int it = 0;
    double res = 0.0;
    bool done = false;
    if (a.mixed) {
+      for (int64_t k = T.lo(nnz) + tid; k < T.hi(nnz); k += THREADS) a.val32[P.nnz_off + k] = (float)val[k];
+      T.bar();
       cg_mixed<THREADS, LPR>(a, P, T, r0, r1, it, res, done);
    }
    else {
@@ -528,37 +447,26 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
       done = res <= a.tol;
       while (!done && it < a.max_it) {
          ++it;
-         double w1[1] = {0.0};
-         block_rows<THREADS, LPR>(r0, r1, A, p, [&](int i, double s) {
-            q[i] = s;
-            w1[0] += p[i] * s;
-         });
+         double w1[1] = {0.0}, dummy = 0.0;
+         block_spmv<THREADS, LPR>(r0, r1, rp, col, val, p, q, p, w1[0], nullptr, nullptr, dummy);
          T.sum(w1);
          const double alpha = rho / w1[0];
          double u2[2] = {0.0, 0.0};
-         double v0[2], v1[2], v2[2], v3[2];
-         for_rows<THREADS>(
-            r0, r1,
-            [&](int i, int j) {
-               v0[j] = r[i];
-               v1[j] = q[i];
-               v2[j] = dinv[i];
-            },
-            [&](int i, int j) {
-               const double ri = v0[j] - alpha * v1[j];
-               r[i] = ri;
-               u2[0] += ri * ri;
-               u2[1] += ri * (v2[j] * ri);
-            });
+         for (int i = r0 + tid; i < r1; i += THREADS) {
+            x[i] += alpha * p[i];
+            const double ri = r[i] - alpha * q[i];
+            r[i] = ri;
+            u2[0] += ri * ri;
+            u2[1] += ri * (dinv[i] * ri);
+         }
          T.sum(u2);
          res = sqrt(u2[0]) / bnorm;
          double rz = u2[1];
          bool restart = false;
          if (res <= a.tol) {
-            for (int i = r0 + tid; i < r1; i += THREADS) x[i] += alpha * p[i];
-            T.bar();
             // FP64 true residual; r <- b - A x either way
-            double w2[1] = {block_residual<THREADS, LPR>(r0, r1, A, x, b, r)};
+            double w2[1] = {0.0}, d2 = 0.0;
+            block_spmv<THREADS, LPR>(r0, r1, rp, col, val, x, nullptr, nullptr, d2, b, r, w2[0]);
             T.sum(w2);
             res = sqrt(w2[0]) / bnorm;
             if (res <= a.tol) {
@@ -573,24 +481,13 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
          }
          const double beta = restart ? 0.0 : rz / rho;
          rho = rz;
-         // (x += alpha p here, where p is read anyway)
-         for_rows<THREADS>(
-            r0, r1,
-            [&](int i, int j) {
-               v0[j] = r[i];
-               v1[j] = dinv[i];
-               v2[j] = p[i];
-               v3[j] = x[i];
-            },
-            [&](int i, int j) {
-               if (!restart) x[i] = v3[j] + alpha * v2[j];
-               p[i] = v1[j] * v0[j] + beta * v2[j];
-            });
+         for (int i = r0 + tid; i < r1; i += THREADS) p[i] = dinv[i] * r[i] + beta * p[i];
          T.bar();
       }
       if (!done && it > 0) {
          // ran out: report the true residual
-         double w2[1] = {block_residual<THREADS, LPR>(r0, r1, A, x, b, q)};
+         double w2[1] = {0.0}, d2 = 0.0;
+         block_spmv<THREADS, LPR>(r0, r1, rp, col, val, x, nullptr, nullptr, d2, b, q, w2[0]);
          T.sum(w2);
          res = sqrt(w2[0]) / bnorm;
       }
@@ -607,21 +504,12 @@ __device__ void solve_problem(const BatchArgs& a, int pid, Team<THREADS>& T)
    }
 }
 
-// What bounds it: the latency of a row's loads times the rows per thread, and
-// what one SM draws from L2.  1024 threads per SM with 64 registers each keep
-// the loads of four entries, or of two rows of a vector pass, in flight; 2048
-// threads with 32 registers spilled or took them one by one.  FP64, default
-// shape, before and now: 400 problems of 1000 to 16000 nodes 48.9 and 42.7 ms,
-// 1000 of 1000 to 4000 22.5 and 16.7; with FP32 inner CG 38.1 and 16.6 of
-// 42.9 and 19.4 (2048 threads with the same loops: 65.9 and 31.4).
-constexpr int kResident = 1024;
-
 // Persistent kernel: a block (CS == 1) or a cluster of CS blocks takes work
 // items from the queue until it is empty.  An item is either up to CS small
 // problems (one per block of the cluster) or one large problem that the
 // whole cluster solves together.
 template <int NEN, int THREADS, int LPR, int CS>
-__global__ void __launch_bounds__(THREADS, kResident / THREADS) batch_kernel(BatchArgs a)
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS) batch_kernel(BatchArgs a)
 {
    __shared__ int s_item;
    __shared__ double sh[3][THREADS / 32];
@@ -659,47 +547,20 @@ __global__ void __launch_bounds__(THREADS, kResident / THREADS) batch_kernel(Bat
    }
 }
 
-// The slices of every problem, one block per problem at a time, one warp per
-// slice: their widths, then (with slice_ptr made from them) their columns, as
-// offsets and absolute; flags an offset that does not fit in 16 bits.
-__global__ void batch_slice_widths(int nprob, const BatchProblem* probs, const int32_t* row_ptr,
-                                   int32_t* width)
+// 16-bit column offsets (column - row, local numbering) of every problem;
+// one block per problem; flags an offset that does not fit
+__global__ void batch_offsets16(int nprob, const BatchProblem* probs, const int32_t* row_ptr,
+                                const int32_t* col, int16_t* d16, int* wide)
 {
-   const int lane = threadIdx.x & 31, w0 = threadIdx.x >> 5, nw = blockDim.x >> 5;
    for (int p = blockIdx.x; p < nprob; p += gridDim.x) {
       const BatchProblem P = probs[p];
       const int32_t* rp = row_ptr + P.rp_off;
-      const int ns = (P.n + 31) >> 5;
-      for (int s = w0; s < ns; s += nw) {
-         const int i = s * 32 + lane;
-         const int w = __reduce_max_sync(0xffffffffu, i < P.n ? rp[i + 1] - rp[i] : 0);
-         if (lane == 0) width[P.slice_off + s] = w;
-      }
-   }
-}
-
-__global__ void batch_slice_columns(int nprob, const BatchProblem* probs, const int32_t* row_ptr,
-                                    const int32_t* col, const int32_t* slice_ptr, int32_t* scol,
-                                    int16_t* soff, int* wide)
-{
-   const int lane = threadIdx.x & 31, w0 = threadIdx.x >> 5, nw = blockDim.x >> 5;
-   for (int p = blockIdx.x; p < nprob; p += gridDim.x) {
-      const BatchProblem P = probs[p];
-      const int32_t* rp = row_ptr + P.rp_off;
-      const int ns = (P.n + 31) >> 5;
-      for (int s = w0; s < ns; s += nw) {
-         const int i = s * 32 + lane;
-         const int c0 = slice_ptr[P.slice_off + s], w = slice_ptr[P.slice_off + s + 1] - c0;
-         const int64_t at = 32 * (int64_t)c0 + lane;
-         const int k0 = i < P.n ? rp[i] : 0, len = i < P.n ? rp[i + 1] - k0 : 0;
-         for (int k = 0; k < w; ++k) {
-            const int c = k < len ? col[P.nnz_off + k0 + k] : min(i, P.n - 1);
-            const int d = k < len ? c - i : 0;
+      for (int i = threadIdx.x; i < P.n; i += blockDim.x)
+         for (int32_t k = rp[i]; k < rp[i + 1]; ++k) {
+            const int d = col[P.nnz_off + k] - i;
             if (d > 32767 || d < -32768) atomicOr(wide, 1);
-            scol[at + 32 * (int64_t)k] = c;
-            soff[at + 32 * (int64_t)k] = (int16_t)d;
+            d16[P.nnz_off + k] = (int16_t)d;
          }
-      }
    }
 }
 
@@ -812,11 +673,7 @@ struct ofg_batch {
    ofg::DBuf<int32_t> order;
    ofg::DBuf<int> queue, bad, iters;
    ofg::DBuf<double> coords;
-   ofg::DBuf<int32_t> elem, code, dof, n2e_ptr, n2e, emap, row_ptr, dpos;
-   // matrices in slices; only one of soff (16-bit offsets) and scol is kept
-   ofg::DBuf<int32_t> slice_ptr, scol;
-   ofg::DBuf<int16_t> soff;
-   ofg::DBuf<double> sval;
+   ofg::DBuf<int32_t> elem, code, dof, n2e_ptr, n2e, emap, row_ptr, col, dpos;
    ofg::DBuf<double> val, b, x, r, p, q, dinv, kel, f, bc, u, res;
    bool have_bc = false;
    int config = -1;  // index into kConfigs; -1: to be chosen (choose_config)
@@ -833,9 +690,10 @@ struct ofg_batch {
    int graph_config = -1;
    int max_it = 0;
    double tol = 0.0;
-   // mixed precision (bits 32): FP32 value copy, FP32 vectors
-   int bits = 64;
-   ofg::DBuf<float> sval32, rl, pl, ql, dl, dinv32;
+   // mixed precision (bits 32): FP32 value copy, 16-bit offsets, FP32 vectors
+   int bits = 64, offsets16 = 0;
+   ofg::DBuf<float> val32, rl, pl, ql, dl, dinv32;
+   ofg::DBuf<int16_t> d16;
    ~ofg_batch()
    {
       if (exec) cudaGraphExecDestroy(exec);
@@ -864,12 +722,9 @@ BatchArgs args_of(ofg_batch* B)
    a.n2e = B->n2e.p;
    a.emap = B->emap.p;
    a.row_ptr = B->row_ptr.p;
+   a.col = B->col.p;
    a.dpos = B->dpos.p;
    a.val = B->val.p;
-   a.slice_ptr = B->slice_ptr.p;
-   a.soff = B->soff.p;
-   a.scol = B->scol.p;
-   a.sval = B->sval.p;
    a.b = B->b.p;
    a.x = B->x.p;
    a.r = B->r.p;
@@ -886,7 +741,9 @@ BatchArgs args_of(ofg_batch* B)
    a.max_it = B->max_it;
    a.tol = B->tol;
    a.mixed = B->bits == 32;
-   a.sval32 = B->sval32.p;
+   a.offsets16 = B->offsets16;
+   a.val32 = B->val32.p;
+   a.d16 = B->d16.p;
    a.rl = B->rl.p;
    a.pl = B->pl.p;
    a.ql = B->ql.p;
@@ -941,17 +798,20 @@ void plan_items(ofg_batch* B, int config, std::vector<int32_t>& order,
 
 // The launch shape of a batch that nobody has chosen one for: 1024 threads,
 // alone or in clusters of 4 or 8, whichever ends first by a model of one
-// iteration, rows per thread plus a constant for its barriers (fitted to 8
-// and 24 problems of up to 4000 and 32000 nodes: 2.7 row steps in one block,
-// 3.3 and 3.55 in clusters), times rows^(1/2) iterations, over the items in
-// their order.  One block per problem leaves the launch waiting for the
-// largest one; with clusters, measured: 24 problems of 1000 to 32000 nodes
-// 60.0 (alone), 21.2 (4), 14.1 ms (8); 192 of them 100.2, 50.2, 53.0; but
-// 192 of 1000 to 4500 5.5, 7.5, 11.8.
+// iteration, rows per thread plus a constant for its barriers (fitted to 24
+// problems of up to 4000 and 32000 nodes: 5.1 row steps in one block, 3.6 and
+// 4.3 in clusters), times rows^(1/2) iterations, over the items in their
+// order.  One block per problem leaves the launch waiting for the largest
+// one; alone, in clusters of 4, of 8, measured: 24 problems of 1000 to 32000
+// nodes 65.0, 24.3, 17.6 ms; 192 of them 102.1, 53.7, 62.5; 400 of 1000 to
+// 16000 48.9, 41.1, 52.1; but 192 of 1000 to 4500 6.5, 8.9, 16.0.  Clusters
+// have to win clearly (kClear): the model leaves out that a full chip shares
+// its L2.
+constexpr double kClear = 0.7;
 int choose_config(ofg_batch* B)
 {
    constexpr int candidate[] = {4, 10, 16};
-   constexpr double barriers[] = {2.7, 3.3, 3.55};
+   constexpr double barriers[] = {5.1, 3.6, 4.3};
    int best = candidate[0];
    double least = 0.0;
    for (int c = 0; c < 3; ++c) {
@@ -972,7 +832,7 @@ int choose_config(ofg_batch* B)
          end = std::max(end, t);
       }
       if (c == 0 || end < least) {
-         least = end;
+         least = c == 0 ? kClear * end : end;
          best = candidate[c];
       }
    }
@@ -1069,42 +929,6 @@ void gather(DBuf<T>& dst, int64_t off, const T* src, int64_t count)
                                stream()));
 }
 
-// the columns of every problem in slices (`slices` pointers in all)
-void build_slices(ofg_batch* B, int64_t slices, const DBuf<int32_t>& col)
-{
-   const int grid = std::min(B->nprob, num_sms() * 4);
-   DBuf<int32_t> width(slices);
-   DBuf<int> wide(1);
-   width.zero();
-   wide.zero();
-   batch_slice_widths<<<grid, 256, 0, stream()>>>(B->nprob, B->d_probs.p, B->row_ptr.p, width.p);
-   count_launch();
-   OFG_LAUNCH_CHECK();
-   std::vector<int32_t> w(slices);
-   width.download(w.data(), slices);
-   std::vector<int32_t> ptr(slices);
-   int64_t positions = 0;   // (no more than nonzeros: below 2^31)
-   for (int64_t s = 0; s < slices; ++s) {   // (a problem's last pointer has width 0)
-      ptr[s] = (int32_t)positions;
-      positions += w[s];
-   }
-   const int64_t total = 32 * positions;
-   B->slice_ptr.alloc(slices);
-   B->slice_ptr.upload(ptr.data(), slices);
-   B->scol.alloc(total);
-   B->soff.alloc(total);
-   B->sval.alloc(total);
-   B->sval.zero();   // the padding stays zero
-   batch_slice_columns<<<grid, 256, 0, stream()>>>(B->nprob, B->d_probs.p, B->row_ptr.p, col.p,
-                                                   B->slice_ptr.p, B->scol.p, B->soff.p, wide.p);
-   count_launch();
-   OFG_LAUNCH_CHECK();
-   int h = 0;
-   wide.download(&h, 1);
-   if (h) B->soff.release();
-   else B->scol.release();
-}
-
 }  // namespace
 }  // namespace ofg
 
@@ -1122,7 +946,6 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
          B->dim = meshes[0]->dim;
          B->nen = meshes[0]->nen;
          std::vector<ofg_matrix*> mats(nprob, nullptr);
-         int64_t slices = 0;
          for (int p = 0; p < nprob; ++p) {
             ofg_mesh* m = meshes[p];
             OFG_REQUIRE(m && m->dim == B->dim, OFG_ERR_ARG, "batch meshes must share one dimension");
@@ -1138,12 +961,10 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
             P.nnz_off = B->nnz;
             P.n2p_off = B->nn + p;
             P.n2e_off = B->ne * m->nen;
-            P.slice_off = slices;
             P.nn = (int32_t)m->nn;
             P.ne = (int32_t)m->ne;
             P.n = (int32_t)mats[p]->n;
 
-            slices += ((P.n + 31) >> 5) + 1;
             B->probs.push_back(P);
             B->nn += m->nn;
             B->ne += m->ne;
@@ -1163,7 +984,7 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
          B->n2e.alloc(B->ne * nen);
          B->emap.alloc(B->ne * nen * nen);
          B->row_ptr.alloc(B->nrows + nprob);
-         DBuf<int32_t> col(B->nnz);
+         B->col.alloc(B->nnz);
          B->dpos.alloc(B->nrows);
          for (int p = 0; p < nprob; ++p) {
             ofg_mesh* m = meshes[p];
@@ -1178,7 +999,7 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
             ensure_emap(A);
             gather(B->emap, P.elem_off * nen * nen, A->emap.p, m->ne * nen * nen);
             gather(B->row_ptr, P.rp_off, A->row_ptr.p, A->n + 1);
-            gather(col, P.nnz_off, A->col.p, A->nnz);
+            gather(B->col, P.nnz_off, A->col.p, A->nnz);
             gather(B->dpos, P.row_off, A->dpos.p, A->n);
          }
          OFG_CUDA(cudaStreamSynchronize(stream()));
@@ -1192,7 +1013,6 @@ int ofg_batch_create(int nprob, ofg_mesh* const* meshes, ofg_batch** out)
          B->items.alloc(nprob);
          B->d_probs.alloc(nprob);
          B->d_probs.upload(B->probs.data(), nprob);
-         build_slices(B, slices, col);
          B->queue.alloc(1);
          B->bad.alloc(1);
          int big = INT32_MAX;
@@ -1365,10 +1185,20 @@ int ofg_batch_set_precision(ofg_batch* B, int bits)
 {
    return guarded("ofg_batch_set_precision", [&] {
       OFG_REQUIRE(B && (bits == 64 || bits == 32), OFG_ERR_ARG, "bits must be 64 or 32");
-      if (bits == 32 && !B->sval32.p) {
+      if (bits == 32 && !B->val32.p) {
+         B->val32.alloc(B->nnz);
          for (auto* v : {&B->rl, &B->pl, &B->ql, &B->dl, &B->dinv32}) v->alloc(B->nrows);
-         B->sval32.alloc(B->sval.n);
-         B->sval32.zero();
+         B->d16.alloc(B->nnz);
+         DBuf<int> wide(1);
+         wide.zero();
+         batch_offsets16<<<std::min(B->nprob, num_sms() * 4), 256, 0, stream()>>>(
+            B->nprob, B->d_probs.p, B->row_ptr.p, B->col.p, B->d16.p, wide.p);
+         count_launch();
+         OFG_LAUNCH_CHECK();
+         int h = 0;
+         wide.download(&h, 1);
+         B->offsets16 = h ? 0 : 1;
+         if (!B->offsets16) B->d16.release();
       }
       if (B->bits != bits) {
          B->bits = bits;

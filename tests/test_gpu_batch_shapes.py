@@ -1,7 +1,7 @@
-"""The batched solver's launch shape chosen from the problems' sizes, and its
-slices of 32 rows: problems of one unknown, around one and many slices, one
-problem far larger than the rest (clusters), many small ones (one block each),
-and columns too far from the row for 16-bit offsets.  Checked as the tuned
+"""The batched solver's launch shape chosen from the problems' sizes: problems
+of one unknown, around a block's rows, one problem far larger than the rest
+(clusters), many small ones (one block each), and columns too far from the row
+for 16-bit offsets.  Checked as the tuned
 shapes are: assembled values bit-exact, solutions to 1e-9, iterations +-2."""
 import numpy as np
 import pytest
@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("bits", [64, 32])
 @pytest.mark.parametrize("sizes", [[2], [2, 3, 6, 7], [33, 2, 34], [5, 120, 9], [40, 90, 41, 42],
                                    [8 + i % 5 for i in range(200)]],
-                         ids=["one", "tiny", "slices", "large", "mixed", "many"])
+                         ids=["one", "tiny", "rows", "large", "mixed", "many"])
 def test_chosen_shape(cuda, sizes, bits):
     B, ref, _ = small_batch(sizes, bc=True)
     B.set_precision(bits)
