@@ -144,7 +144,7 @@ struct ofg_prec {
    ofg::DBuf<double> t;
    ofg::DBuf<int> status;    // bounded-wait failures (bit 0: timeout, bit 1: wave)
    ofg::SweepPlan fwd, bwd;
-   ofg::WavePlan wfwd, wbwd;  // both on, or both off
+   ofg::WavePlan wfwd, wbwd;  // both on and of the same `ext`, or both off
    ofg::DBuf<int32_t> tpos;  // D-ILU: transposed position of each lower entry
    ofg::DBuf<double> dot;    // (r, z) of the last backward sweep that was asked for it
    int grid = 0;             // blocks of the persistent factorisation sweep launch

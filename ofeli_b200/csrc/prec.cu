@@ -5,9 +5,10 @@
 //
 // Two forms of the sweeps.  Matrices whose rows form long grid lines with at
 // most three couplings to the line itself and the one before (structured
-// meshes in natural order) take the wavefront of wave.cu, both directions or
-// none; every other matrix (unstructured files, short or ragged lines) takes
-// the sweeps of this file.
+// meshes in natural order) take the wavefront of wave.cu, both directions in
+// the same form or none; every other matrix (unstructured files, short or
+// ragged lines, couplings to far lines on one side only) takes the sweeps of
+// this file.
 //
 // Sweep scheduling here.  Rows keep OFELI's natural order, so the preconditioner
 // is the reference's own.  Rows are cut into strands: maximal runs of
@@ -1209,8 +1210,12 @@ void prec_setup(ofg_prec* P)
       P->t.alloc(n > 0 ? n : 1);
       P->dot.alloc(1);
       const std::vector<int8_t> cf = host_chain(A, true), cb = host_chain(A, false);
+      // (one form for both: with E slots the vector between the sweeps is not
+      // scaled by the pivots yet, without them it is; a pattern that is not
+      // symmetric may have E slots in one direction only)
       const bool wave = wave_build(A, true, cf.data(), ilu ? P->tpos.p : nullptr, P->wfwd) &&
-                        wave_build(A, false, cb.data(), nullptr, P->wbwd);
+                        wave_build(A, false, cb.data(), nullptr, P->wbwd) &&
+                        P->wfwd.ext == P->wbwd.ext;
       if (!wave) {
          P->wfwd = WavePlan();
          P->wbwd = WavePlan();
@@ -1272,9 +1277,10 @@ void prec_apply_device(ofg_prec* P, const double* r, double* z, double* rz, cons
    if (P->wfwd.on) {
       // (the results of a sweep are waited for in memory only with E slots:
       // then each sweep clears the other's buffer)
-      wave_solve(P, true, r, P->t.p, P->wbwd.ext ? z : nullptr, nullptr, nullptr, skip);
+      const bool ext = P->wfwd.ext;
+      wave_solve(P, true, r, P->t.p, ext ? z : nullptr, nullptr, nullptr, skip);
       const bool dot = rz && r != z;
-      wave_solve(P, false, P->t.p, z, P->wfwd.ext ? P->t.p : nullptr, dot ? r : nullptr, rz, skip);
+      wave_solve(P, false, P->t.p, z, ext ? P->t.p : nullptr, dot ? r : nullptr, rz, skip);
       return;
    }
    const bool dilu = (P->type != OFG_SSOR);

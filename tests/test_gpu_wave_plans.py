@@ -1,0 +1,82 @@
+"""What the two plans of the wavefront sweeps (csrc/wave.cu) have to agree on
+and leave alone: patterns that are not symmetric, blocks that go on from group
+to group, values written through the device pointer, right-hand sides that
+hold the sweeps' own marker.  Checked against the oracle; a row's result
+carries a handful of roundings of its own and those of the rows before, damped
+by the diagonally dominant triangle: 1e-13."""
+import numpy as np
+import pytest
+
+from ofeli_b200 import ofeli as F
+from oracle import oracle as O
+from test_gpu_wave import cube, square
+
+pytestmark = pytest.mark.gpu
+
+
+def assembled(mesh, seed=3):
+    dim, xy, elem, code = mesh
+    dof, n = O.number_equations(code)
+    rp, ci = O.node_graph(elem, dim + 1, dof, n)
+    rng = np.random.default_rng(seed)
+    k = rng.uniform(0.3, 3.0, elem.size // (dim + 1))
+    a, _ = O.assemble(dim, xy, elem, dof, code, n, rp, ci, k=k, f=np.ones(code.size),
+                      bc=np.zeros(code.size))
+    return rp, ci, a, n
+
+
+def rows_of(rp):
+    return np.repeat(np.arange(1, rp.size), np.diff(rp))
+
+
+def from_triplets(row, col, val, n):
+    order = np.lexsort((col, row))
+    rp = np.zeros(n + 1, np.int64)
+    rp[1:] = np.cumsum(np.bincount(row - 1, minlength=n))
+    return rp, col[order], val[order]
+
+
+def one_more(mesh, at):
+    """The mesh's matrix and one entry far from the diagonal."""
+    rp, ci, a, n = assembled(mesh)
+    i, j = at(n)
+    return from_triplets(np.append(rows_of(rp), i), np.append(ci, j), np.append(a, 0.5), n) + (n,)
+
+
+def one_sided(mesh, far, upper):
+    """Without the couplings of `far` columns or more to one side."""
+    rp, ci, a, n = assembled(mesh)
+    r = rows_of(rp)
+    keep = ci - r < far if upper else r - ci < far
+    return from_triplets(r[keep], ci[keep], a[keep], n) + (n,)
+
+
+def check(P, ptype, rp, ci, a, b):
+    idv, piv = O.prec_setup(ptype, rp, ci, a)
+    if ptype == F.ILU_PREC:
+        assert np.array_equal(P.getPivot(), piv)
+    z0 = O.prec_apply(ptype, rp, ci, a, idv, piv, b)
+    z = P.solve(b)
+    assert np.abs(z - z0).max() <= 1e-13 * np.abs(z0).max()
+    return z
+
+
+UNSYMMETRIC = {
+    "far_upper": lambda: one_more(square(64, 64), lambda n: (5, n - 1)),
+    "far_lower": lambda: one_more(square(64, 64), lambda n: (n - 1, 5)),
+    "planes_lower": lambda: one_sided(cube(12), 11 * 11, True),
+    "planes_upper": lambda: one_sided(cube(12), 11 * 11, False),
+}
+
+
+@pytest.mark.parametrize("ptype", [F.ILU_PREC, F.SSOR_PREC])
+@pytest.mark.parametrize("name", sorted(UNSYMMETRIC))
+def test_unsymmetric_patterns(cuda, name, ptype):
+    rp, ci, a, n = UNSYMMETRIC[name]()
+    b = np.random.default_rng(4).uniform(-1, 1, n)
+    P = F.Prec(F.SpMatrix(rp, ci, a), ptype)
+    z = check(P, ptype, rp, ci, a, b)
+    assert np.array_equal(P.solve(b), z)
+    x = b.copy()
+    P.solve(x, x)
+    assert np.array_equal(x, z)
