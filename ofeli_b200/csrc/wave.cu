@@ -564,7 +564,10 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
             if (!EXT) {
                const int tt = lane & 7;
 #pragma unroll 1
-               for (int cc = 0; cc < kTileChunks; ++cc) {
+               // (no chunk past the group's: nothing would clear lane 0's
+               // places there, and where the block's next group hands a line
+               // to lane 0 they must read as not written yet)
+               for (int cc = 0; cc < kTileChunks && tl * kTileChunks + cc < nch; ++cc) {
                   const int t = (tl * kTileChunks + cc) * kWaveF + tt;
 #pragma unroll
                   for (int q = 0; q < 8; ++q) {

@@ -80,3 +80,41 @@ def test_unsymmetric_patterns(cuda, name, ptype):
     x = b.copy()
     P.solve(x, x)
     assert np.array_equal(x, z)
+
+
+def blocks(count):
+    """Grids of 40 lines of 9 to 71 rows side by side, uncoupled."""
+    parts = [assembled(square(41, 10 + 61 * q // (count - 1)), seed=q) for q in range(count)]
+    off = np.cumsum([0] + [p[3] for p in parts])
+    nz = np.cumsum([0] + [p[1].size for p in parts])
+    rp = np.concatenate([[0]] + [p[0][1:] + z for p, z in zip(parts, nz)])
+    return rp, np.concatenate([p[1] + o for p, o in zip(parts, off)]), np.concatenate(
+        [p[2] for p in parts]), int(off[-1])
+
+
+# more groups than a GPU has SMs, so that blocks go on from group to group; the
+# first group's steps end inside a tile (with 9, 17 and 29 chunks of eight)
+TALL = {
+    "tall_36": lambda: assembled(square(4710, 36)),
+    "tall_100": lambda: assembled(square(4710, 100)),
+    "tall_200": lambda: assembled(square(4700, 200)),
+    "blocks": lambda: blocks(110),
+}
+
+
+@pytest.mark.parametrize("ptype", [F.ILU_PREC, F.SSOR_PREC])
+@pytest.mark.parametrize("name", sorted(TALL))
+def test_blocks_go_on_from_group_to_group(cuda, name, ptype):
+    rp, ci, a, n = TALL[name]()
+    b = np.random.default_rng(4).uniform(-1, 1, n)
+    A = F.SpMatrix(rp, ci, a)
+    P = F.Prec(A, ptype)
+    z = check(P, ptype, rp, ci, a, b)
+    piv = P.getPivot()
+    x = np.empty(n)
+    for q in range(200):
+        if q % 10 == 0:
+            P.setMatrix()
+            assert np.array_equal(P.getPivot(), piv)
+        P.solve(b, x)
+        assert np.array_equal(x, z)
