@@ -16,6 +16,9 @@ struct ofg_matrix {
    ofg::DBuf<int32_t> row_ptr, col;
    ofg::DBuf<double> val;
    uint64_t version = 1;  // bumped whenever values change
+   // the value array was handed out (ofg_matrix_device_arrays): the caller may
+   // write through the pointer at any time, without a new version
+   bool exposed = false;
 
    // diagonal position of every row (OFELI's id[i]-1); -1 if absent
    ofg::DBuf<int32_t> dpos;
@@ -172,6 +175,9 @@ namespace ofg {
 // matrix.cu
 void ensure_dpos(ofg_matrix* A);
 void ensure_sell(ofg_matrix* A);
+// the same from the values as they are now, also where they were written
+// through the pointer that ofg_matrix_device_arrays gave out
+void refresh_sell(ofg_matrix* A);
 void ensure_sell32(ofg_matrix* A);
 void ensure_sell_bf16(ofg_matrix* A);
 // new values into the FP64, FP32 and BF16 SELL copies in one pass, *inexact

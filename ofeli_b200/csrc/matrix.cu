@@ -517,6 +517,12 @@ void ensure_sell(ofg_matrix* A)
    }
 }
 
+void refresh_sell(ofg_matrix* A)
+{
+   if (A->exposed) A->sell_version = 0;
+   ensure_sell(A);
+}
+
 void ensure_sell32(ofg_matrix* A)
 {
    if (A->sell_ready && A->sell_version != A->version && A->sell_val32.n == A->sell_val.n) {
@@ -773,6 +779,7 @@ int ofg_matrix_device_arrays(const ofg_matrix* A, const int32_t** row_ptr, const
       if (values) {
          *values = A->val.p;
          const_cast<ofg_matrix*>(A)->version++;  // caller may write through it
+         const_cast<ofg_matrix*>(A)->exposed = true;
       }
    });
 }

@@ -1182,7 +1182,11 @@ void prec_setup(ofg_prec* P)
    int big = INT32_MAX;
    bad.upload(&big, 1);
    const int invert = (P->type == OFG_SSOR) ? 0 : 1;
-   if (P->wfwd.on) wave_diagonal(P, invert, bad.p);
+   // (the wavefront's set-up reads the values from the SELL copy)
+   if (P->wfwd.on) {
+      refresh_sell(A);
+      wave_diagonal(P, invert, bad.p);
+   }
    else if (n) {
       diag_setup<<<grid_for(n, 256), 256, 0, stream()>>>(n, A->dpos.p, A->val.p, P->pivot.p, invert,
                                                          bad.p);
@@ -1205,7 +1209,8 @@ void prec_setup(ofg_prec* P)
          OFG_LAUNCH_CHECK();
       }
    }
-   if (!P->status.p) {
+   const bool first = !P->status.p;
+   if (first) {
       P->status.alloc(1);
       P->t.alloc(n > 0 ? n : 1);
       P->dot.alloc(1);
@@ -1234,7 +1239,7 @@ void prec_setup(ofg_prec* P)
    if (P->wfwd.on) {
       if (P->wfwd.ext) fill_sentinel(P->t.p, n);
       if (ilu) {
-         ensure_sell(A);
+         if (first) refresh_sell(A);
          wave_factor(P);
          check_status(P);
       }

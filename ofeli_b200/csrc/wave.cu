@@ -1323,8 +1323,7 @@ bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpo
 
 void wave_diagonal(ofg_prec* P, int invert, int* bad)
 {
-   ofg_matrix* A = P->A;
-   ensure_sell(A);
+   const ofg_matrix* A = P->A;
    wave_diag<<<grid_for(A->n, 256), 256, 0, stream()>>>(A->n, A->row_ptr.p, A->dpos.p, A->sell_ptr.p,
                                                         A->sell_val.p, P->pivot.p, invert, bad);
    count_launch();

@@ -4,9 +4,13 @@ to group, values written through the device pointer, right-hand sides that
 hold the sweeps' own marker.  Checked against the oracle; a row's result
 carries a handful of roundings of its own and those of the rows before, damped
 by the diagonally dominant triangle: 1e-13."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
+from ofeli_b200 import capi
 from ofeli_b200 import ofeli as F
 from oracle import oracle as O
 from test_gpu_wave import cube, square
@@ -118,3 +122,35 @@ def test_blocks_go_on_from_group_to_group(cuda, name, ptype):
             assert np.array_equal(P.getPivot(), piv)
         P.solve(b, x)
         assert np.array_equal(x, z)
+
+
+class Values:
+    """The matrix's device value array as a tensor's source."""
+
+    def __init__(self, A):
+        p = ctypes.c_void_p()
+        capi.call("ofg_matrix_device_arrays", A._h, None, None, ctypes.byref(p))
+        self.__cuda_array_interface__ = dict(shape=(A.nnz,), typestr="<f8",
+                                             data=(p.value, False), version=3)
+
+
+@pytest.mark.parametrize("ptype", [F.ILU_PREC, F.SSOR_PREC])
+@pytest.mark.parametrize("mesh", [square(64, 64), cube(12)], ids=["square", "cube"])
+def test_values_written_through_the_device_pointer(cuda, mesh, ptype):
+    """setMatrix(), and a new Prec, take the values that are there, whenever
+    they were written, with copies of earlier ones made in between."""
+    rp, ci, a, n = assembled(mesh)
+    rng = np.random.default_rng(6)
+    b = rng.uniform(-1, 1, n)
+    A = F.SpMatrix(rp, ci, a)
+    values = torch.as_tensor(Values(A), device="cuda:0")
+    P = F.Prec(A, ptype)
+    check(P, ptype, rp, ci, a, b)
+    for _ in range(3):
+        A.Mult(b)
+        a = a * rng.uniform(0.95, 1.0, a.size)
+        values.copy_(torch.from_numpy(a))
+        torch.cuda.synchronize()
+        P.setMatrix()
+        z = check(P, ptype, rp, ci, a, b)
+        assert np.array_equal(F.Prec(A, ptype).solve(b), z)
