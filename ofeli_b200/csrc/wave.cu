@@ -388,7 +388,7 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
                                            WaveRun<wave_slots(MODE)>& R)
 {
    double cn[kWaveF];
-   bool have = same_tile, special = false;
+   bool have = same_tile, stop = false;
    int m = 0;
 #pragma unroll
    for (int s = 0; s < kWaveF; ++s) {
@@ -411,9 +411,10 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
       // spread over the steps, so that no step waits for it
       if (s == 4) m = max4(cn[0], cn[1], cn[2], cn[3]);
       if (s == 5) m = max(m, max4(cn[4], cn[5], cn[6], cn[7]));
-      if (s == 6) special = __any_sync(0xffffffffu, m >= 0x7ff00000);
+      // (one answer for the warp, of the lanes' own barrier tests too)
+      if (s == 6) stop = __any_sync(0xffffffffu, !have || m >= 0x7ff00000);
    }
-   R.go = next_ok && have && !special;
+   R.go = next_ok && !stop;
 #pragma unroll
    for (int q = 0; q < kWaveF; ++q) R.op.c[q] = cn[q];
 }
