@@ -592,8 +592,10 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          double* src = g.edge + (first ? ein : 0);
          for (int tl = 0; first && tl < ntile; ++tl) {
             const ChunkAt<MODE> at(tiles, tl * kTileChunks);
+            // (one answer for the warp: the polls below are votes)
             if (tiles + tl >= Sh::NT &&
-                !wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u, &sh.stop, g.status))
+                !__all_sync(0xffffffffu, wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u,
+                                                  &sh.stop, g.status)))
                break;
             const int i = tl * kWaveTile + lane - sm1;
             // (past the group's chunks nothing clears the place again)
