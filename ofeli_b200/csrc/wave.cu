@@ -205,6 +205,7 @@ struct WaveShared {
    double c[NT * kTileChunks][kWaveF / 2 * kWaveCPitch];
    double z[NT * kTileChunks][kWaveF * kWavePitch];
    unsigned long long full[NT], empty[NT];
+   unsigned fed;   // tiles whose copies have been issued
    int group, stop;
 };
 
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       sh.stop = 0;
+      sh.fed = 0;
    }
    for (int i = threadIdx.x; i < Sh::NT * kTileChunks * kWaveF * kWavePitch; i += blockDim.x)
       (&sh.z[0][0])[i] = wave_sentinel();
@@ -552,9 +554,13 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          }
          for (int tl = 0; tl < ntile; ++tl) {
             const ChunkAt<MODE> at(tiles, tl * kTileChunks);
+            // (one answer for the warp: a tile's copies are issued by all
+            // lanes or none)
             if (tiles + tl >= Sh::NT &&
-                !wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u, &sh.stop, g.status))
+                !__all_sync(0xffffffffu, wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u,
+                                                  &sh.stop, g.status)))
                break;
+            if (lane == 0) sh.fed = tiles + tl + 1;
             const uint32_t bar = smem_u32(&sh.full[at.tile]);
             if (lane == 0) {
                constexpr uint32_t bytes = kWaveTile * NS * 32 * sizeof(double);
@@ -831,9 +837,17 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
       }
       tiles += ntile;
    }
-   // a block that gave up may have copies in flight: they end within
-   // microseconds; its shared memory stays until they have
-   if (sh.stop) __nanosleep(1000000);
+   // a block that gave up may have copies in flight into its shared memory,
+   // which has to stay until they have arrived: the last tiles fed (one a
+   // place of the ring) are waited for, with a limit
+   if (w == 1 && sh.stop) {
+      const unsigned fed = sh.fed;
+      const unsigned long long t0 = global_ns();
+      for (unsigned t = fed > Sh::NT ? fed - Sh::NT : 0; t < fed; ++t)
+         while (!mbar_test(smem_u32(&sh.full[t % Sh::NT]), (t / Sh::NT) & 1u) &&
+                global_ns() - t0 <= kWaveLimitNs) {
+         }
+   }
    if (threadIdx.x == 0) {
       __threadfence();
       if (atomicAdd(&g.ticket[2], 1) == (int)gridDim.x - 1) {
