@@ -111,6 +111,11 @@ __device__ __forceinline__ bool wave_empty(double v)
    return (unsigned long long)__double_as_longlong(v) == kSentinelBits;
 }
 __device__ __forceinline__ double wave_sentinel() { return __longlong_as_double((long long)kSentinelBits); }
+// a value that came in from outside: the sentinel's own bits become another NaN
+__device__ __forceinline__ double wave_plain(double v)
+{
+   return wave_empty(v) ? __longlong_as_double(0x7FF8000000000000ll) : v;
+}
 
 __device__ __forceinline__ unsigned long long global_ns()
 {
@@ -426,12 +431,13 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
 // storing warps see its results arrive (the z tile holds the sentinel
 // before), which also tells that the operands of those steps are free; a
 // barrier arrival with its fence costs 100 to 200 cycles a chunk.
-// lo, hi: the steps in which the fast form may be used.
+// lo, hi: the steps in which the fast form may be used; flagged: this lane's
+// right-hand sides arrive on their own, the sentinel in their places until
+// then (the others come with the tile, whatever bits they hold).
 template <int MODE>
 __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, unsigned tiles,
-                                             int nch, int lane, bool carry, const LineInfo& li,
-                                             double* edge_out,
-                                             int lo, int hi)
+                                             int nch, int lane, bool carry, bool flagged,
+                                             const LineInfo& li, double* edge_out, int lo, int hi)
 {
    WaveRun<wave_slots(MODE)> R;
    R.z = R.u1 = R.u2 = 0.0;
@@ -460,7 +466,7 @@ __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, 
          bool missing = false;
 #pragma unroll
          for (int q = 0; q < kWaveF; ++q) missing = missing || wave_empty(R.op.c[q]);
-         if (!__any_sync(0xffffffffu, missing)) break;
+         if (!__any_sync(0xffffffffu, flagged && missing)) break;
          if ((spins & 255u) == 0 && __any_sync(0xffffffffu, wave_give_up(w0, &sh.stop, status)))
             break;
       }
@@ -543,7 +549,8 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          const int lo = g.clean ? 0 : __reduce_max_sync(0xffffffffu, li.shift);
          const int hi = g.clean ? INT_MAX
                                 : __reduce_min_sync(0xffffffffu, li.len ? li.shift + li.len : INT_MAX);
-         wave_compute<MODE>(sh, g.status, tiles, nch, lane, first && lane == 0, li, edge_out, lo, hi);
+         const bool carry = first && lane == 0;
+         wave_compute<MODE>(sh, g.status, tiles, nch, lane, carry, EXT || carry, li, edge_out, lo, hi);
       }
       else if (w == 1) {
          // ---------------------------------------------------------- feed
@@ -806,6 +813,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
                v[k] = 0.0;
                if (!wave_empty(r.a[k])) pend |= 1u << k;
             }
+            double c = FWD ? wave_plain(r.b) : r.b;   // (backward it is multiplied first)
             const unsigned long long w0 = global_ns();
             for (unsigned spins = 1; pend; ++spins) {
 #pragma unroll
@@ -816,7 +824,6 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
                   if (!wave_empty(v[k])) pend &= ~(1u << k);
                if ((spins & 255u) == 0 && wave_give_up(w0, &sh.stop, g.status)) break;
             }
-            double c = r.b;
             if (MODE == W_FACTOR) {
 #pragma unroll
                for (int k = 0; k < kExt; ++k)
@@ -1053,7 +1060,7 @@ __global__ void __launch_bounds__(256) wave_fill(FillArgs f)
 #pragma unroll
                   for (int q = 0; q < kExt; ++q)
                      if (f.eoff[(size_t)l * kExt + q] == c - rho) {
-                        e[q] = vs;
+                        e[q] = wave_plain(vs);
                         et[q] = vt;
                      }
                }

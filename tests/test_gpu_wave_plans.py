@@ -154,3 +154,35 @@ def test_values_written_through_the_device_pointer(cuda, mesh, ptype):
         P.setMatrix()
         z = check(P, ptype, rp, ci, a, b)
         assert np.array_equal(F.Prec(A, ptype).solve(b), z)
+
+
+MARKER = np.array([0x7FF4DEADBEEF0001], np.uint64).view(np.float64)[0]
+
+
+@pytest.mark.parametrize("ptype", [F.ILU_PREC, F.SSOR_PREC])
+@pytest.mark.parametrize("mesh", [square(64, 64), cube(12)], ids=["square", "cube"])
+def test_the_sweeps_own_marker_is_a_nan_like_any_other(cuda, mesh, ptype):
+    """In the right-hand side or in the matrix: the results are those of a
+    NaN in its place."""
+    rp, ci, a, n = assembled(mesh)
+    b = np.random.default_rng(6).uniform(-1, 1, n)
+    A = F.SpMatrix(rp, ci, a)
+    P = F.Prec(A, ptype)
+    for at in ([0], [n // 2, n // 2 + 1], [n - 1], list(range(n))):
+        c, d = b.copy(), b.copy()
+        c[at], d[at] = MARKER, np.nan
+        z, z0 = P.solve(c), P.solve(d)
+        assert np.isnan(z[at]).all()
+        assert np.array_equal(z, z0, equal_nan=True)
+    r = n // 2
+    row = np.arange(rp[r], rp[r + 1])          # a lower, the diagonal and an upper entry
+    for k in (row[0], row[ci[row] == r + 1][0], row[-1]):
+        z = []
+        for v in (MARKER, np.nan):
+            c = a.copy()
+            c[k] = v
+            A.set_values(c)
+            P.setMatrix()
+            z.append(P.solve(b))
+        assert np.isnan(z[0]).any()
+        assert np.array_equal(z[0], z[1], equal_nan=True)
