@@ -114,9 +114,26 @@ struct SweepPlan {
 // to 32, the coefficients in the order the steps read them.
 constexpr int kWaveExt = 4;        // entries a row may have in earlier groups
 // The wavefront is taken when a line has at least kWaveMinLine rows on
-// average and a step at least kWaveMinLanes active lanes.
+// average and a step at least kWaveMinLanes active lanes.  On 2-D grids it is
+// the faster form wherever these hold, long and thin ones included (us per CG
+// iteration with ILU, strands of prec.cu / wavefront: 8 lines of 8 rows
+// 65 / 37, 5 of 16 78 / 38, 5 of 1024 134 / 112, 8 of 2048 235 / 191, 32 of
+// 8192 977 / 680, 1000 of 9 4380 / 171).
 constexpr int64_t kWaveMinLine = 8;
 constexpr int64_t kWaveMinLanes = 4;
+// With entries in earlier groups (3-D) a row along a line costs the wavefront
+// more (its right-hand side waits for the plane before, then the chunk), a
+// line in a plane the strands; both pay per plane.  It is taken where
+//    (rows a line)^2 planes <= kWaveLongLine (lines a plane)^2,
+// a plane being a run of lines each coupled to the one before.  Measured on
+// 316 boxes of 16 to 1500 rows, 8 to 128 lines, 3 to 128 planes (CG with ILU
+// and SSOR, strands / wavefront, us per iteration with ILU): 63^3 1.30 times
+// as fast, 127^3 1.45, 256 x 32 x 16 182 / 177; refused: 1024 x 16 x 64
+// 540 / 671, 1024 x 128 x 16 589 / 634, 512 x 64 x 64 601 / 677.  Near the
+// line one form or the other is up to 14 % faster; worst on the wavefront's
+// side are deep boxes whose lines fill the strands' segments of 32 rows
+// (32 x 32 x 128: 492 / 531).
+constexpr double kWaveLongLine = 800.0;
 struct WavePlan {
    bool on = false, fwd = true;
    bool ext = false;          // some row has entries in earlier groups

@@ -1305,6 +1305,12 @@ bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpo
    g_line.push_back(nl);
    const int64_t tiles = (int64_t)tile_g.size();
    if (n < kWaveMinLanes * steps || tiles * kWaveTile * 32 * 4 > INT_MAX) return false;
+   if (p.ext) {
+      // see kWaveLongLine
+      const double planes = (double)std::count(g_edge.begin(), g_edge.end(), -1);
+      const double rows = (double)n / nl, lines = nl / planes;
+      if (rows * rows * planes > kWaveLongLine * lines * lines) return false;
+   }
    p.ngroups = (int)g_line.size() - 1;
    p.tiles = tiles;
    auto put = [&](DBuf<int32_t>& d, const std::vector<int32_t>& h) {

@@ -186,3 +186,33 @@ def test_the_sweeps_own_marker_is_a_nan_like_any_other(cuda, mesh, ptype):
             z.append(P.solve(b))
         assert np.isnan(z[0]).any()
         assert np.array_equal(z[0], z[1], equal_nan=True)
+
+
+def box(rows, lines, planes, seed=5):
+    """A box of unknowns coupled as the Kuhn cube's: 14 neighbours."""
+    dims, st = (rows, lines, planes), (1, rows, rows * lines)
+    idx = np.arange(rows * lines * planes)
+    at = [idx // s % d for s, d in zip(st, dims)]
+    r, c = [idx], [idx]
+    for q in range(1, 8):
+        step = [(q >> k) & 1 for k in range(3)]
+        ok = np.all([a + s < d for a, s, d in zip(at, step, dims)], axis=0)
+        to = idx[ok] + sum(s * t for s, t in zip(step, st))
+        r += [idx[ok], to]
+        c += [to, idx[ok]]
+    r, c = np.concatenate(r), np.concatenate(c)
+    a = np.where(r == c, 16.0, -np.random.default_rng(seed).uniform(0.5, 1.0, r.size))
+    return from_triplets(r + 1, c + 1, a, idx.size) + (idx.size,)
+
+
+@pytest.mark.parametrize("ptype", [F.ILU_PREC, F.SSOR_PREC])
+@pytest.mark.parametrize("dims", [(80, 8, 8), (81, 8, 8), (40, 12, 6), (33, 34, 5), (500, 6, 3),
+                                  (9, 40, 7)], ids=str)
+def test_boxes_on_both_sides_of_the_line(cuda, dims, ptype):
+    """Boxes of short lines take the wavefront, those of long ones the strands
+    (80 and 81 rows are next to it for 8 lines and 8 planes)."""
+    rp, ci, a, n = box(*dims)
+    b = np.random.default_rng(4).uniform(-1, 1, n)
+    P = F.Prec(F.SpMatrix(rp, ci, a), ptype)
+    z = check(P, ptype, rp, ci, a, b)
+    assert np.array_equal(P.solve(b), z)
