@@ -210,8 +210,7 @@ struct WaveShared {
    double c[NT * kTileChunks][kWaveF / 2 * kWaveCPitch];
    double z[NT * kTileChunks][kWaveF * kWavePitch];
    unsigned long long full[NT], empty[NT];
-   unsigned fed;   // tiles whose copies have been issued
-   int group, stop;
+   int group, stop, unfed;  // unfed: tiles that a block that gave up left out
 };
 
 // Where chunk `ch` of a group lies in shared memory; tiles: those of the
@@ -386,7 +385,7 @@ struct WaveRun {
 // The coefficients are read kAhead steps ahead and the next chunk's
 // right-hand sides and readiness early in this one, so that the chunks follow
 // each other without a wait.
-template <int MODE, bool FAST>
+template <int MODE, bool EXT, bool FAST>
 __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int next, bool same_tile,
                                            uint32_t next_bar, unsigned next_phase, bool next_ok,
                                            int j0, int len, int lane, bool carry,
@@ -394,7 +393,7 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
                                            WaveRun<wave_slots(MODE)>& R)
 {
    double cn[kWaveF];
-   bool have = same_tile, stop = false;
+   bool have = same_tile, special = false;
    int m = 0;
 #pragma unroll
    for (int s = 0; s < kWaveF; ++s) {
@@ -417,10 +416,15 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
       // spread over the steps, so that no step waits for it
       if (s == 4) m = max4(cn[0], cn[1], cn[2], cn[3]);
       if (s == 5) m = max(m, max4(cn[4], cn[5], cn[6], cn[7]));
-      // (one answer for the warp, of the lanes' own barrier tests too)
-      if (s == 6) stop = __any_sync(0xffffffffu, !have || m >= 0x7ff00000);
+      if (s == 6) special = __any_sync(0xffffffffu, m >= 0x7ff00000);
+      // (one answer for the warp, of the lanes' own tests of the barrier; its
+      // place measured at 512^2 and 63^3, us per CG + ILU iteration: without
+      // a vote 166.0 and 328.2, after step 1 167.6 and 330, 2 167.8 and 331,
+      // 3 167.6 and 331, 5 166.4 and 330, 7 170.0 and 328.4, within the vote
+      // on special values 168.5 and 330)
+      if (s == (EXT ? 7 : 5)) have = __all_sync(0xffffffffu, have);
    }
-   R.go = next_ok && !stop;
+   R.go = next_ok && have && !special;
 #pragma unroll
    for (int q = 0; q < kWaveF; ++q) R.op.c[q] = cn[q];
 }
@@ -431,13 +435,14 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
 // storing warps see its results arrive (the z tile holds the sentinel
 // before), which also tells that the operands of those steps are free; a
 // barrier arrival with its fence costs 100 to 200 cycles a chunk.
-// lo, hi: the steps in which the fast form may be used; flagged: this lane's
-// right-hand sides arrive on their own, the sentinel in their places until
-// then (the others come with the tile, whatever bits they hold).
-template <int MODE>
+// lo, hi: the steps in which the fast form may be used.  The right-hand sides
+// of lane 0 where it carries a line, with E slots those of all lanes, arrive
+// on their own, the sentinel in their places until then; the others come with
+// the tile, whatever bits they hold.
+template <int MODE, bool EXT>
 __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, unsigned tiles,
-                                             int nch, int lane, bool carry, bool flagged,
-                                             const LineInfo& li, double* edge_out, int lo, int hi)
+                                             int nch, int lane, bool carry, const LineInfo& li,
+                                             double* edge_out, int lo, int hi)
 {
    WaveRun<wave_slots(MODE)> R;
    R.z = R.u1 = R.u2 = 0.0;
@@ -447,7 +452,7 @@ __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, 
    auto steps = [&](auto fast, int ch) {
       const ChunkAt<MODE> at(tiles, ch), nx(tiles, ch + 1);
       const int t0 = ch * kWaveF;
-      wave_steps<MODE, decltype(fast)::value>(
+      wave_steps<MODE, EXT, decltype(fast)::value>(
          sh, at.slot, nx.slot, nx.tile == at.tile, smem_u32(&sh.full[nx.tile]), nx.phase,
          ch + 1 < nch && t0 + kWaveF >= lo && t0 + 2 * kWaveF <= hi && !special, t0 - li.shift,
          li.len, lane, carry, edge_out ? edge_out + t0 : nullptr, R);
@@ -466,7 +471,7 @@ __device__ __forceinline__ void wave_compute(WaveShared<MODE>& sh, int* status, 
          bool missing = false;
 #pragma unroll
          for (int q = 0; q < kWaveF; ++q) missing = missing || wave_empty(R.op.c[q]);
-         if (!__any_sync(0xffffffffu, flagged && missing)) break;
+         if (!__any_sync(0xffffffffu, (EXT || carry) && missing)) break;
          if ((spins & 255u) == 0 && __any_sync(0xffffffffu, wave_give_up(w0, &sh.stop, status)))
             break;
       }
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       sh.stop = 0;
-      sh.fed = 0;
+      sh.unfed = 0;
    }
    for (int i = threadIdx.x; i < Sh::NT * kTileChunks * kWaveF * kWavePitch; i += blockDim.x)
       (&sh.z[0][0])[i] = wave_sentinel();
@@ -549,8 +554,8 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
          const int lo = g.clean ? 0 : __reduce_max_sync(0xffffffffu, li.shift);
          const int hi = g.clean ? INT_MAX
                                 : __reduce_min_sync(0xffffffffu, li.len ? li.shift + li.len : INT_MAX);
-         const bool carry = first && lane == 0;
-         wave_compute<MODE>(sh, g.status, tiles, nch, lane, carry, EXT || carry, li, edge_out, lo, hi);
+         wave_compute<MODE, EXT>(sh, g.status, tiles, nch, lane, first && lane == 0, li, edge_out, lo,
+                                 hi);
       }
       else if (w == 1) {
          // ---------------------------------------------------------- feed
@@ -565,9 +570,10 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
             // lanes or none)
             if (tiles + tl >= Sh::NT &&
                 !__all_sync(0xffffffffu, wave_bar(smem_u32(&sh.empty[at.tile]), at.phase ^ 1u,
-                                                  &sh.stop, g.status)))
+                                                  &sh.stop, g.status))) {
+               if (lane == 0) sh.unfed = ntile - tl;
                break;
-            if (lane == 0) sh.fed = tiles + tl + 1;
+            }
             const uint32_t bar = smem_u32(&sh.full[at.tile]);
             if (lane == 0) {
                constexpr uint32_t bytes = kWaveTile * NS * 32 * sizeof(double);
@@ -848,7 +854,7 @@ __global__ void __launch_bounds__(wave_threads(EXT), 1) wave_sweep(WaveArgs g)
    // which has to stay until they have arrived: the last tiles fed (one a
    // place of the ring) are waited for, with a limit
    if (w == 1 && sh.stop) {
-      const unsigned fed = sh.fed;
+      const unsigned fed = tiles - sh.unfed;
       const unsigned long long t0 = global_ns();
       for (unsigned t = fed > Sh::NT ? fed - Sh::NT : 0; t < fed; ++t)
          while (!mbar_test(smem_u32(&sh.full[t % Sh::NT]), (t / Sh::NT) & 1u) &&
