@@ -804,9 +804,12 @@ void plan_items(ofg_batch* B, int config, std::vector<int32_t>& order,
 // order.  One block per problem leaves the launch waiting for the largest
 // one; alone, in clusters of 4, of 8, measured: 24 problems of 1000 to 32000
 // nodes 65.0, 24.3, 17.6 ms; 192 of them 102.1, 53.7, 62.5; 400 of 1000 to
-// 16000 48.9, 41.1, 52.1; but 192 of 1000 to 4500 6.5, 8.9, 16.0.  Clusters
-// have to win clearly (kClear): the model leaves out that a full chip shares
-// its L2.
+// 16000 48.9, 41.1, 52.1; but 192 of 1000 to 4500 6.5, 8.9, 16.0, and one
+// problem of 196 unknowns 0.30, 0.49, 0.52, of 784 0.77, 0.96, 1.02 (up to
+// 1024 rows a cluster has no fewer row steps), of 1156 1.32, 1.22, 1.23, of
+// 3721 4.74, 2.67, 2.41.  FP32 is alike (0.37, 0.55, 0.59; 0.86, 1.11, 1.17;
+// 1.19, 1.24, 1.30; 4.03, 2.60, 2.49).  Clusters have to win clearly (kClear):
+// the model leaves out that a full chip shares its L2.
 constexpr double kClear = 0.7;
 int choose_config(ofg_batch* B)
 {
@@ -825,7 +828,12 @@ int choose_config(ofg_batch* B)
       double end = 0.0;
       for (const BatchItem& w : items) {
          const double n = B->probs[order[w.first]].n;   // (the largest of a group)
-         const double steps = w.big ? n / (1024.0 * cs) + barriers[c] : n / 1024.0 + barriers[0];
+         // whole row steps in 2-D: a thread without a row waits at the barriers
+         // all the same.  (In 3-D, with 15 entries a row and 24 elements a
+         // node, a share of the threads' work counts: 512 unknowns 0.55 ms in
+         // one block, 0.50 in a cluster of 4, 729 0.75 and 0.63.)
+         const double rows = n / (1024.0 * (w.big ? cs : 1));
+         const double steps = (B->nen == 3 ? std::ceil(rows) : rows) + barriers[w.big ? c : 0];
          const double t = busy.top() + std::sqrt(n) * steps;
          busy.pop();
          busy.push(t);
