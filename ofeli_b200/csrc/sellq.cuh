@@ -78,7 +78,6 @@ constexpr int kHoist = 1;
 // register budget: 65536 / (256 * kQuadBlocks)), and the grid of the
 // kernel chains they are part of.
 constexpr int kQuadBlocks = 8;
-constexpr int kValueUnroll = 1;
 
 // The four rows r0 .. r0+3 of a uniform slice: w positions, the offset of
 // position k from tp[k].  The values of kHoist positions are loaded before
@@ -128,7 +127,7 @@ __device__ __forceinline__ float4 value_quad(const int2* __restrict__ tp, int w,
                                              const float* __restrict__ x, int r0)
 {
    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll kValueUnroll
+#pragma unroll 1
    for (int k = 0; k < w; ++k) {
       const int2 e = __ldg(tp + k);
       const float a = __int_as_float(e.x);
