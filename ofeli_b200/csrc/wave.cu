@@ -44,6 +44,7 @@
 // for belongs to a block that is already running.  Every wait is bounded.
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <type_traits>
 
 #include "internal.cuh"
@@ -1216,11 +1217,10 @@ bool wave_build(ofg_matrix* A, bool fwd, const int8_t* chain, const int32_t* tpo
    p.fwd = fwd;
    if (n < 1) return false;
    std::vector<int32_t> line(1, 0);
-   for (int64_t r = 1; r < n; ++r)
-      if (!chain[r]) {
-         line.push_back((int32_t)r);
-         if ((int64_t)line.size() * kWaveMinLine > n + kWaveMinLine) return false;
-      }
+   for (const int8_t* q = chain + 1; (q = (const int8_t*)std::memchr(q, 0, chain + n - q)); ++q) {
+      line.push_back((int32_t)(q - chain));
+      if ((int64_t)line.size() * kWaveMinLine > n + kWaveMinLine) return false;
+   }
    line.push_back((int32_t)n);
    const int nl = (int)line.size() - 1;
    p.line.alloc(line.size());
