@@ -419,11 +419,13 @@ __device__ __forceinline__ void wave_steps(WaveShared<MODE>& sh, int slot, int n
       if (s == 5) m = max(m, max4(cn[4], cn[5], cn[6], cn[7]));
       if (s == 6) special = __any_sync(0xffffffffu, m >= 0x7ff00000);
       // (one answer for the warp, of the lanes' own tests of the barrier; its
-      // place measured at 512^2 and 63^3, us per CG + ILU iteration: without
-      // a vote 166.0 and 328.2, after step 1 167.6 and 330, 2 167.8 and 331,
-      // 3 167.6 and 331, 5 166.4 and 330, 7 170.0 and 328.4, within the vote
-      // on special values 168.5 and 330)
-      if (s == (EXT ? 7 : 5)) have = __all_sync(0xffffffffu, have);
+      // place measured, us per CG + ILU iteration at 512^2 and 63^3: without a
+      // vote 166.0 and 328.2, after step 1 167.6 and 330, 2 167.8 and 331, 3
+      // 167.6 and 331, 5 166.4 and 330, 7 170.0 and 328.4, within the vote on
+      // special values 168.5 and 330; set-up with the factorisation at 2047^2:
+      // without 1042, after step 1 to 5 1078, 1058, 1075, 1051, 1076, 6 1050,
+      // 7 1053)
+      if (s == (EXT ? 7 : MODE == W_FACTOR ? 6 : 5)) have = __all_sync(0xffffffffu, have);
    }
    R.go = next_ok && have && !special;
 #pragma unroll
