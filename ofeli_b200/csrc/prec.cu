@@ -7,8 +7,8 @@
 // most three couplings to the line itself and the one before (structured
 // meshes in natural order) take the wavefront of wave.cu, both directions in
 // the same form or none; every other matrix (unstructured files, short or
-// ragged lines, couplings to far lines on one side only) takes the sweeps of
-// this file.
+// ragged lines, couplings to far lines on one side only, boxes of long lines)
+// takes the sweeps of this file.
 //
 // Sweep scheduling here.  Rows keep OFELI's natural order, so the preconditioner
 // is the reference's own.  Rows are cut into strands: maximal runs of
